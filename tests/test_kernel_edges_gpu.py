@@ -1,0 +1,52 @@
+"""The attention, router and row kernels at the sizes where their tiling can go wrong: remainders of tiles, the smallest
+and largest of their ranges, both sides of every rule that picks a variant."""
+import pytest
+import torch
+
+from uttt_b200 import ops
+from uttt_b200.ops._ext import load
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _status_ok():
+    st = load(required=True).gemm_status(torch.zeros(1, device=DEV))
+    assert int(st[0].item()) == 0, f"a tensor-core kernel reported a timed-out wait (code {int(st[0])})"
+
+
+def _rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+
+
+# One query; one tile less and more than a row block; a window that starts inside a tile, of one key, and wider than the
+# keys; history that ends inside a tile; query blocks of one and of two tiles (few and many heads); unmasked with
+# remainders; a negative and a zero scale.
+@pytest.mark.parametrize("b,h,lq,lk,hd,window,causal,scale", [
+    (1, 2, 1, 1, 64, None, True, None), (1, 3, 1, 700, 64, 256, True, None), (2, 3, 127, 127, 96, None, True, None),
+    (1, 2, 129, 300, 128, 64, True, None), (1, 2, 260, 260, 64, 1, True, None), (2, 40, 300, 777, 96, 513, True, None),
+    (2, 45, 256, 256, 64, 2048, True, None), (3, 30, 257, 257, 128, None, False, None), (1, 2, 100, 640, 64, None, False, None),
+    (1, 2, 200, 333, 64, 128, True, -0.2), (1, 2, 200, 333, 64, 128, True, 0.0)])
+def test_attention_tile_edges(b, h, lq, lk, hd, window, causal, scale):
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(lq + lk)
+    q, do = (torch.randn(b, lq, h, hd, generator=gen, device=DEV).bfloat16() for _ in range(2))
+    k, v = (torch.randn(b, lk, h, hd, generator=gen, device=DEV).bfloat16() for _ in range(2))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    out = ops.swa_attention(*leaves, window, causal=causal, scale=scale)
+    grads = torch.autograd.grad(out, leaves, do)
+    torch.cuda.synchronize()
+    _status_ok()
+    exact = [t.detach().double().requires_grad_() for t in leaves]
+    s = torch.einsum("bqhd,bkhd->bhqk", exact[0], exact[1]) * (hd ** -0.5 if scale is None else scale)
+    if causal:
+        qp, kp = torch.arange(lk - lq, lk, device=DEV)[:, None], torch.arange(lk, device=DEV)[None]
+        s = s.masked_fill((kp > qp) | (kp <= qp - (window or lk + 1)), float("-inf"))
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), exact[2])
+    want_grads = torch.autograd.grad(want, exact, do.double())
+    # bf16 results and bf16 probabilities / dS between the products: 2^-9 relative each, a few of them in a row
+    for name, got, ref_ in zip(("out", "dq", "dk", "dv"), (out, *grads), (want, *want_grads)):
+        if float(ref_.abs().max()) < 1e-9:                       # a single visible key: dS is zero but for rounding of D
+            assert float(got.float().abs().max()) < 2e-2, name
+        else:
+            assert _rel(got, ref_) < 1e-2, (name, _rel(got, ref_))

@@ -4,16 +4,20 @@
 //   causal: key j visible to query i (absolute position p = lk - lq + i) iff j <= p and j > p - window.
 //   non-causal (window ignored): every key visible (full attention inside one view).
 //
-// One CTA = one (batch, head, 128-query tile).  It walks the 64-key tiles of its band:
-//   warp 8 / lane 0 : TMA producer   K_j, V_j -> 2-stage 128B-swizzled ring
-//   warp 9 / lane 0 : MMA issuer     S_j = Q K_j^T (double-buffered in TMEM), O_j = P_j V_j
-//   warps 0-7       : softmax        two threads per query row (its TMEM lane), one per 32-column half of the
-//                                    tile: one TMEM read of S_j, row maximum exchanged through shared memory,
-//                                    P_j written back to shared memory (reusing K_j's slot) as the bf16 A
-//                                    operand of the second MMA.  O is accumulated in TMEM by the tensor core
-//                                    relative to a per-row reference maximum that moves only when the running
-//                                    maximum exceeds it by 8 (log2 units); only then O is rescaled in TMEM.
-// Two CTAs are resident per SM so one CTA's softmax overlaps the other's MMAs.
+// One CTA = one (batch, head) and one or two 128-query tiles.  It walks the 128-key tiles of the union of their bands:
+//   warps 0-3, 4-7  : softmax of query tile 0 / 1, one thread per query row (= TMEM lane): the whole row of S_j is read
+//                     into registers, P_j = 2^(S_j - ref) goes back to tensor memory as bf16 over S_j and is the A
+//                     operand of the second product.  O is accumulated in TMEM relative to a per-row reference
+//                     maximum that moves only when the running maximum exceeds it by 8 (log2 units); only then O is
+//                     rescaled in TMEM.
+//   warp 8 / lane 0 : TMA producer   K_j, V_j -> 128B-swizzled rings
+//   warp 9 / lane 0 : MMA issuer     per step and query tile: O += P_{j-1} V_{j-1}, then S_j = Q K_j^T
+// The two query tiles alternate: while the tensor core works for one, the other's softmax warps run, and each K/V tile
+// is fetched once for 256 queries.  Bound by the chain S -> softmax -> P -> MMA of a tile (tensor pipe a third busy,
+// exponential unit under half); a step of 128 keys pays its hand-overs once where a step of 64 paid them twice.
+// Measured against two 128-query CTAs per SM with steps of 64 keys and two threads to a row: 275 -> 152 us at 4 x 16
+// heads x 96, 2048 queries on 4096 keys, window 2048; 109 -> 72 us at 12 x 12 heads x 64, 1024 tokens unmasked.  Steps of
+// 64 keys with two S buffers per query tile in this layout: 180 and 83 us.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -32,62 +36,80 @@ struct SwaParams {
   int lq, lk, heads, hd;
   int window;       // 0 = unlimited
   int causal;
-  float scale_log2; // softmax scale * log2(e)
+  int tiles;        // 128-query tiles per CTA: 1 or 2
+  int flip;         // the softmax scale is negative: S is negated and scale_log2 holds |scale| * log2(e)
+  float scale_log2; // |softmax scale| * log2(e), > 0
   __nv_bfloat16* out;
   float* lse;       // [b, h, lq], natural log of the row sums of exp(scale * s)
   int* status;
 };
 
-constexpr int kQ = 128;   // queries per CTA
-constexpr int kKV = 64;   // keys per tile
-constexpr int kStageBytes = 32 * 1024;   // K slot (16 KB, later reused for P) + V slot (16 KB)
-constexpr int kQBytes = 32 * 1024;
-constexpr int kXchgBytes = 2 * 2 * kQ * 4;   // row maxima exchanged between the two column halves, double-buffered
-constexpr int kAttnSmem = kQBytes + 2 * kStageBytes + kXchgBytes + 160 + 1024;
+constexpr int kQ = 128;   // queries per tile
+constexpr int kKV = 128;  // keys per tile
+constexpr int kSlabBytes = 128 * 128;        // 128 rows x 64 bf16, one 128-byte swizzle row each
+// Three warpgroups at 168 registers each; the softmax ones take 208 (a row of S lives in registers), the third gives
+// its share up: 2 x 208 + 80 <= 3 x 168.
+constexpr int kThreads = 384;
+constexpr int kSoftmaxRegs = 208, kOtherRegs = 80;
+static_assert(2 * kSoftmaxRegs + kOtherRegs <= 3 * 168, "more registers than the block is launched with");
 constexpr float kRescaleThreshold = 8.f;     // log2 units: P stays below 2^8 between rescales
 
-// Rendezvous of the two warps that share a TMEM lane quarter (one per column half): an mbarrier with 64 arrivals
-// per phase, waited on with the bounded wait so that a warp whose partner gave up cannot hang.
-__device__ __forceinline__ bool pair_sync(uint32_t bar, uint32_t use, int* status) {
-  ptx::mbar_arrive(bar);
-  return ptx::mbar_wait(bar, use & 1, status, 19);
-}
+template <int HD>
+struct SwaCfg {
+  static constexpr int KB = (HD + 63) / 64;                // 64-wide slabs along the head dimension
+  static constexpr int kTile = KB * kSlabBytes;
+  static constexpr int kStages = HD == 64 ? 4 : 2;         // K and V ring depth
+  static constexpr int kBars = 2 * kTile + 2 * kStages * kTile;
+  static constexpr int kSmem = kBars + 256 + 1024;
+};
 
 template <int HD>
-__global__ void __launch_bounds__(320, 2) swa_fwd_kernel(const __grid_constant__ CUtensorMap tq,
+__global__ void __launch_bounds__(kThreads, 1) swa_fwd_kernel(const __grid_constant__ CUtensorMap tq,
                                                          const __grid_constant__ CUtensorMap tk,
                                                          const __grid_constant__ CUtensorMap tv, SwaParams p) {
+  using C = SwaCfg<HD>;
+  constexpr int KB = C::KB, ST = C::kStages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - ptx::smem_u32(smem_raw));
-  const uint32_t q_smem = base;
-  auto k_smem = [&](int s) { return base + kQBytes + s * kStageBytes; };
-  auto v_smem = [&](int s) { return base + kQBytes + s * kStageBytes + 16 * 1024; };
-  float* xchg = reinterpret_cast<float*>(gen + kQBytes + 2 * kStageBytes);      // [2 buffers][2 halves][128 rows]
-  const uint32_t bars = base + kQBytes + 2 * kStageBytes + kXchgBytes;
-  // barrier slots
-  const uint32_t q_full = bars;
-  auto k_full = [&](int s) { return bars + 8 + 8 * s; };
-  auto v_full = [&](int s) { return bars + 24 + 8 * s; };
-  auto empty = [&](int s) { return bars + 40 + 8 * s; };
-  auto s_done = [&](int s) { return bars + 56 + 8 * s; };
-  auto p_ready = [&](int s) { return bars + 72 + 8 * s; };
-  const uint32_t o_done = bars + 88;
-  auto pair_bar = [&](int quarter) { return bars + 96 + 8 * quarter; };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + kQBytes + 2 * kStageBytes + kXchgBytes + 128);
+  auto q_smem = [&](int s) { return base + s * C::kTile; };
+  auto k_smem = [&](int st) { return base + (2 + st) * C::kTile; };
+  auto v_smem = [&](int st) { return base + (2 + ST + st) * C::kTile; };
+  const uint32_t bars = base + C::kBars;
+  auto q_full = [&](int s) { return bars + 8 * s; };
+  auto s_done = [&](int s) { return bars + 16 + 8 * s; };
+  auto p_ready = [&](int s) { return bars + 32 + 8 * s; };
+  auto o_done = [&](int s) { return bars + 48 + 8 * s; };
+  auto k_full = [&](int st) { return bars + 64 + 8 * st; };
+  auto v_full = [&](int st) { return bars + 96 + 8 * st; };
+  auto k_empty = [&](int st) { return bars + 128 + 8 * st; };
+  auto v_empty = [&](int st) { return bars + 160 + 8 * st; };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + C::kBars + 192);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
-  const int q0 = qt * kQ;
+  const int warp = ptx::warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  // the last query tiles see the most keys when the history is short: they are issued first
+  const int blocks_q = (p.lq + kQ * p.tiles - 1) / (kQ * p.tiles);
+  const int head = blockIdx.x % p.heads, batch = blockIdx.y;
+  const int q00 = (blocks_q - 1 - blockIdx.x / p.heads) * kQ * p.tiles;
   const int shift = p.lk - p.lq;          // absolute position of query 0
-  // key tile range of this query tile
-  int first_key = 0, last_key = p.lk - 1;
-  if (p.causal) {
-    last_key = min(p.lk - 1, shift + q0 + kQ - 1);
-    if (p.window > 0) first_key = max(0, shift + q0 - p.window + 1);
+  // key tile range of each query tile
+  int lo_t[2] = {0, 0}, hi_t[2] = {0, 0};
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const int q0 = q00 + s * kQ;
+    if (s < p.tiles && q0 < p.lq) {
+      int first_key = 0, last_key = p.lk - 1;
+      if (p.causal) {
+        last_key = min(p.lk - 1, shift + q0 + kQ - 1);
+        if (p.window > 0) first_key = max(0, shift + q0 - p.window + 1);
+      }
+      lo_t[s] = first_key / kKV;
+      hi_t[s] = last_key / kKV + 1;
+    }
   }
-  const int t0 = first_key / kKV;
-  const int nt = last_key / kKV - t0 + 1;
+  const bool two = hi_t[1] > lo_t[1];
+  const int t0 = lo_t[0];                                   // the first query tile's band starts first
+  const int nt = (two ? hi_t[1] : hi_t[0]) - t0;            // and the second one's ends last
 
   {
     __shared__ int prior_failure;
@@ -96,203 +118,201 @@ __global__ void __launch_bounds__(320, 2) swa_fwd_kernel(const __grid_constant__
     if (prior_failure != 0) return;
   }
   if (threadIdx.x == 0) {
-    ptx::mbar_init(q_full, 1);
     for (int s = 0; s < 2; ++s) {
-      ptx::mbar_init(k_full(s), 1);
-      ptx::mbar_init(v_full(s), 1);
-      ptx::mbar_init(empty(s), 1);
+      ptx::mbar_init(q_full(s), 1);
       ptx::mbar_init(s_done(s), 1);
-      ptx::mbar_init(p_ready(s), 256);
+      ptx::mbar_init(p_ready(s), 128);
+      ptx::mbar_init(o_done(s), 1);
     }
-    ptx::mbar_init(o_done, 1);
-    for (int qd = 0; qd < 4; ++qd) ptx::mbar_init(pair_bar(qd), 64);
+    for (int st = 0; st < ST; ++st) {
+      ptx::mbar_init(k_full(st), 1);
+      ptx::mbar_init(v_full(st), 1);
+      ptx::mbar_init(k_empty(st), 1);
+      ptx::mbar_init(v_empty(st), 1);
+    }
     ptx::mbar_fence_init();
     ptx::tma_prefetch_desc(&tq);
     ptx::tma_prefetch_desc(&tk);
     ptx::tma_prefetch_desc(&tv);
   }
   if (warp == 8) {
-    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), 256);
+    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), 512);
     ptx::tmem_relinquish();
   }
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::tc_fence_after_sync();
-  const uint32_t tmem = *tmem_slot;
-  const uint32_t tmem_s0 = tmem;          // S buffers: columns [0,64) and [64,128)
-  const uint32_t tmem_o = tmem + 128;     // O: columns [128, 128 + HD), accumulated by the tensor core
+  const uint32_t tmem = ptx::warp_uniform(*tmem_slot);
+  auto tmem_s = [&](int s) { return tmem + s * 128; };           // S_j (fp32), overwritten by P_j (bf16, 64 columns)
+  auto tmem_o = [&](int s) { return tmem + 256 + s * 128; };
 
-  constexpr int KB = (HD + 63) / 64;      // 64-wide blocks along the head dimension
   constexpr uint32_t idesc_s = ptx::make_instr_desc(kQ, kKV, 0, 0);
   constexpr uint32_t idesc_o = ptx::make_instr_desc(kQ, HD, 0, 1);
   bool ok = true;
 
-  if (warp == 8 && lane == 0) {
-    // ================= producer =================
-    ptx::mbar_expect_tx(q_full, KB * kQ * 128);
-    for (int kb = 0; kb < KB; ++kb)
-      ptx::tma_load_3d(q_smem + kb * (kQ * 128), &tq, q_full, head * HD + kb * 64, q0, batch);
-    for (int j = 0; j < nt && ok; ++j) {
-      int s = j & 1;
-      if (j >= 2) ok = ptx::mbar_wait(empty(s), ((j >> 1) - 1) & 1, p.status, 11);
-      if (!ok) break;
-      int key0 = (t0 + j) * kKV;
-      ptx::mbar_expect_tx(k_full(s), KB * kKV * 128);
-      for (int kb = 0; kb < KB; ++kb)
-        ptx::tma_load_3d(k_smem(s) + kb * (kKV * 128), &tk, k_full(s), head * HD + kb * 64, key0, batch);
-      ptx::mbar_expect_tx(v_full(s), KB * kKV * 128);
-      for (int kb = 0; kb < KB; ++kb)
-        ptx::tma_load_3d(v_smem(s) + kb * (kKV * 128), &tv, v_full(s), head * HD + kb * 64, key0, batch);
-    }
-  } else if (warp == 9 && lane == 0) {
-    // ================= MMA issuer =================
-    auto issue_s = [&](int j) -> bool {
-      int s = j & 1;
-      if (!ptx::mbar_wait(k_full(s), (j >> 1) & 1, p.status, 12)) return false;
-      ptx::tc_fence_after_sync();
-#pragma unroll
-      for (int k = 0; k < HD / 16; ++k) {
-        uint64_t da = ptx::make_smem_desc(q_smem + (k >> 2) * (kQ * 128) + (k & 3) * 32, 16, 1024);
-        uint64_t db = ptx::make_smem_desc(k_smem(s) + (k >> 2) * (kKV * 128) + (k & 3) * 32, 16, 1024);
-        ptx::mma_bf16_ss(tmem_s0 + s * 64, da, db, idesc_s, k > 0 ? 1u : 0u);
+  // each role's code stays inside the branch that sets its register share
+  if (warp >= 8) {
+    ptx::reg_dec<kOtherRegs>();
+    if (warp == 8 && lane == 0) {
+      // ================= producer =================
+      auto load = [&](uint32_t dst, const CUtensorMap* map, uint32_t bar, int row) {
+        ptx::mbar_expect_tx(bar, C::kTile);
+        for (int kb = 0; kb < KB; ++kb)
+          ptx::tma_load_3d(dst + kb * kSlabBytes, map, bar, head * HD + kb * 64, row, batch);
+      };
+      load(q_smem(0), &tq, q_full(0), q00);
+      for (int j = 0; j < nt && ok; ++j) {
+        const int st = j % ST;
+        if (j >= ST) ok = ptx::mbar_wait(k_empty(st), (j / ST - 1) & 1, p.status, 11);
+        if (!ok) break;
+        load(k_smem(st), &tk, k_full(st), (t0 + j) * kKV);
+        if (j == 0 && two) load(q_smem(1), &tq, q_full(1), q00 + kQ);
+        if (j >= ST) ok = ptx::mbar_wait(v_empty(st), (j / ST - 1) & 1, p.status, 12);
+        if (!ok) break;
+        load(v_smem(st), &tv, v_full(st), (t0 + j) * kKV);
       }
-      ptx::mma_commit(s_done(s));
-      return true;
-    };
-    ok = ptx::mbar_wait(q_full, 0, p.status, 13);
-    if (ok) ok = issue_s(0);
-    for (int j = 0; j < nt && ok; ++j) {
-      int s = j & 1;
-      // S_{j+1} runs on the tensor core while the softmax threads work on S_j: its TMEM buffer was
-      // drained before p_ready(j-1), and its K tile lands only after P_{j-1} V_{j-1} released the stage.
-      if (j + 1 < nt) ok = issue_s(j + 1);
-      if (!ok) break;
-      ok = ptx::mbar_wait(p_ready(s), (j >> 1) & 1, p.status, 14);
-      if (!ok) break;
-      ok = ptx::mbar_wait(v_full(s), (j >> 1) & 1, p.status, 15);
-      if (!ok) break;
-      ptx::tc_fence_after_sync();
+    } else if (warp == 9) {
+      // ================= MMA issuer =================
+      // S_j overwrites P_{j-1}: the product that reads P_{j-1} was issued before it by this thread, and the tensor core
+      // runs them in order.  For the same reason "S_j is complete" says that O has received P_{j-1} V_{j-1}.
+      const bool leader = ptx::elect_one();
+      for (int j = 0; j <= nt && ok; ++j) {
 #pragma unroll
-      for (int k = 0; k < kKV / 16; ++k) {
-        uint64_t da = ptx::make_smem_desc(k_smem(s) + k * 32, 16, 1024);                 // P_j (K-major)
-        uint64_t db = ptx::make_smem_desc(v_smem(s) + k * 2048, kKV * 128, 1024);        // V_j (N-major slabs)
-        ptx::mma_bf16_ss(tmem_o, da, db, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+        for (int s = 0; s < 2; ++s) {
+          const int first = lo_t[s] - t0, last = hi_t[s] - t0 - 1;       // this query tile's steps
+          if (s == 1 && !two) continue;
+          if (j - 1 >= first && j - 1 <= last) {
+            const int st = (j - 1) % ST;
+            ok = ptx::warp_wait(p_ready(s), (j - 1 - first) & 1, p.status, 13) &&
+                 ptx::warp_wait(v_full(st), ((j - 1) / ST) & 1, p.status, 14);
+            if (!ok) break;
+            ptx::tc_fence_after_sync();
+#pragma unroll
+            for (int k = 0; k < kKV / 16; ++k) {
+              const uint64_t db = ptx::make_smem_desc(v_smem(st) + k * 2048, kSlabBytes, 1024);   // V_j (N-major slabs)
+              if (leader) ptx::mma_bf16_ts(tmem_o(s), tmem_s(s) + k * 8, db, idesc_o, (j - 1 > first || k > 0) ? 1u : 0u);
+            }
+            if (leader && j - 1 == last) ptx::mma_commit(o_done(s));
+          }
+          if (j >= first && j <= last) {
+            const int st = j % ST;
+            if (j == first) ok = ptx::warp_wait(q_full(s), 0, p.status, 15);
+            ok = ok && ptx::warp_wait(k_full(st), (j / ST) & 1, p.status, 16);
+            if (!ok) break;
+            ptx::tc_fence_after_sync();
+#pragma unroll
+            for (int k = 0; k < HD / 16; ++k) {
+              const uint64_t da = ptx::make_smem_desc(q_smem(s) + (k >> 2) * kSlabBytes + (k & 3) * 32, 16, 1024);
+              const uint64_t db = ptx::make_smem_desc(k_smem(st) + (k >> 2) * kSlabBytes + (k & 3) * 32, 16, 1024);
+              if (leader) ptx::mma_bf16_ss(tmem_s(s), da, db, idesc_s, k > 0 ? 1u : 0u);
+            }
+            if (leader) ptx::mma_commit(s_done(s));
+          }
+        }
+        if (!ok) break;
+        if (leader && j < nt) ptx::mma_commit(k_empty(j % ST));
+        if (leader && j > 0) ptx::mma_commit(v_empty((j - 1) % ST));
       }
-      ptx::mma_commit(o_done);
-      ptx::mma_commit(empty(s));
     }
-  }
-
-  // ================= softmax (warps 0-7): thread = (query row, half of the 64 key columns) =================
-  // O stays in TMEM and is accumulated by the tensor core relative to a reference maximum m_ref per row; the
-  // reference moves (and O, l are rescaled) only when the running maximum exceeds it by kRescaleThreshold.
-  if (warp < 8) {
-    const int half = warp >> 2;
+  } else {
+    ptx::reg_inc<kSoftmaxRegs>();
+    // ================= softmax (warps 0-7): thread = query row =================
+    const int s = warp >> 2;
     const int quarter = warp & 3;
+    const int q0 = q00 + s * kQ;
     const int r = quarter * 32 + lane;            // query row inside the tile == TMEM lane
     const int qpos = shift + q0 + r;              // absolute position
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    float m_ref = -INFINITY, l_part = 0.f;
+    const int first = s ? lo_t[1] : lo_t[0], n = s ? hi_t[1] - lo_t[1] : hi_t[0] - lo_t[0];
+    float m_ref = -INFINITY, l_run = 0.f;
 
-    for (int j = 0; j < nt; ++j) {
-      int s = j & 1;
-      if (!ptx::mbar_wait(s_done(s), (j >> 1) & 1, p.status, 16)) { ok = false; break; }
+    for (int j = 0; j < n; ++j) {
+      if (!ptx::mbar_wait(s_done(s), j & 1, p.status, 17)) { ok = false; break; }
       ptx::tc_fence_after_sync();
-      const int key0 = (t0 + j) * kKV + half * 32;
-      bool need_mask = (key0 + 32 > p.lk);
+      uint32_t raw[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) ptx::tmem_ld_32x32(tmem_s(s) + lane_base + c * 32, raw[c]);
+      ptx::tmem_ld_wait();
+      if (p.flip) {
+#pragma unroll
+        for (int i = 0; i < 128; ++i) raw[i >> 5][i & 31] ^= 0x80000000u;
+      }
+      const int key0 = (first + j) * kKV;
+      bool need_mask = (key0 + kKV > p.lk);
       if (p.causal) {
-        need_mask = need_mask || (key0 + 31 > shift + q0);
+        need_mask = need_mask || (key0 + kKV - 1 > shift + q0);
         if (p.window > 0) need_mask = need_mask || (key0 <= shift + q0 + kQ - 1 - p.window);
       }
-      uint32_t raw[32];
-      ptx::tmem_ld_32x32(tmem_s0 + s * 64 + lane_base + half * 32, raw);
-      ptx::tmem_ld_wait();
-      float x[32];
-      float mx = -INFINITY;
+      if (need_mask) {
+        // visible columns of this row: [lo, lo + span]
+        int hi = p.lk - 1 - key0, lo = 0;
+        if (p.causal) {
+          hi = min(hi, qpos - key0);
+          if (p.window > 0) lo = max(0, qpos - key0 - p.window + 1);
+        }
+        if (hi < lo) { lo = 1 << 20; hi = lo; }
+        const uint32_t span = (uint32_t)(hi - lo);
+#pragma unroll
+        for (int i = 0; i < 128; ++i)
+          if ((uint32_t)(i - lo) > span) raw[i >> 5][i & 31] = 0xff800000u;
+      }
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
-        x[i] = __uint_as_float(raw[i]) * p.scale_log2;
-        if (need_mask) {
-          const int kp = key0 + i;
-          bool vis = kp < p.lk;
-          if (p.causal) {
-            vis = vis && (kp <= qpos);
-            if (p.window > 0) vis = vis && (kp > qpos - p.window);
-          }
-          if (!vis) x[i] = -INFINITY;
-        }
-        mx = fmaxf(mx, x[i]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) m4[c] = fmaxf(m4[c], __uint_as_float(raw[c][i]));
       }
-      // row maximum over both halves
-      float* xb = xchg + (j & 1) * 2 * kQ;
-      xb[half * kQ + r] = mx;
-      if (!pair_sync(pair_bar(quarter), (uint32_t)j, p.status)) { ok = false; break; }
-      mx = fmaxf(mx, xb[(half ^ 1) * kQ + r]);
+      const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
       const bool move_ref = mx > m_ref + kRescaleThreshold;     // also true for the first visible key (m_ref = -inf)
       const float new_ref = move_ref ? mx : m_ref;
-      const float factor = move_ref ? exp2f(m_ref - new_ref) : 1.f;    // m_ref = -inf -> 0
-      const float m_use = (new_ref == -INFINITY) ? 0.f : new_ref;
-      float rs = 0.f;
-      uint8_t* prow = gen + (k_smem(s) - base) + r * 128;
+      if (j > 0 && __any_sync(0xffffffffu, move_ref)) {
+        const float factor = move_ref ? exp2f(m_ref - new_ref) : 1.f;    // m_ref = -inf -> 0
+        l_run *= factor;
 #pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        float e[8];
+        for (int c = 0; c < HD / 32; ++c) {
+          uint32_t o[32];
+          ptx::tmem_ld_32x32(tmem_o(s) + lane_base + c * 32, o);
+          ptx::tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          e[i] = exp2f(x[ch * 8 + i] - m_use);
-          rs += e[i];
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+          ptx::tmem_st_32x32(tmem_o(s) + lane_base + c * 32, o);
         }
-        uint4 u;
-        __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) h2[i] = __floats2bfloat162_rn(e[2 * i], e[2 * i + 1]);
-        const int chunk = half * 4 + ch;
-        *reinterpret_cast<uint4*>(prow + ((chunk ^ (r & 7)) << 4)) = u;
       }
-      l_part = l_part * factor + rs;
       m_ref = new_ref;
-      // O may be touched only after P_{j-1} V_{j-1} has finished; P_j V_j starts after p_ready(j)
-      if (j > 0) {
-        if (!ptx::mbar_wait(o_done, (j - 1) & 1, p.status, 17)) { ok = false; break; }
-        if (__any_sync(0xffffffffu, move_ref)) {
-          ptx::tc_fence_after_sync();
+      const float neg = (new_ref == -INFINITY) ? 0.f : -new_ref;
+      const float2 neg2 = make_float2(neg, neg), scale2 = make_float2(p.scale_log2, p.scale_log2);
+      float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-          for (int c = 0; c < HD / 32; ++c) {
-            if ((c & 1) != half) continue;
-            uint32_t o[32];
-            ptx::tmem_ld_32x32(tmem_o + lane_base + c * 32, o);
-            ptx::tmem_ld_wait();
+      for (int c = 0; c < 2; ++c) {
+        uint32_t w[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-            ptx::tmem_st_32x32(tmem_o + lane_base + c * 32, o);
-          }
-          ptx::tmem_st_wait();
+        for (int i = 0; i < 32; ++i) {
+          const int col = c * 64 + 2 * i;
+          float2 x = make_float2(__uint_as_float(raw[col >> 5][col & 31]), __uint_as_float(raw[col >> 5][(col & 31) + 1]));
+          x = __ffma2_rn(x, scale2, neg2);
+          x.x = exp2f(x.x);
+          x.y = exp2f(x.y);
+          rs[i & 1] = __fadd2_rn(rs[i & 1], x);
+          w[i] = ptx::pack_bf16x2(x);
         }
+        ptx::tmem_st_32x32(tmem_s(s) + lane_base + c * 32, w);
       }
-      ptx::fence_proxy_async();          // make the generic-proxy writes of P visible to the tensor core
+      l_run += (rs[0].x + rs[0].y) + (rs[1].x + rs[1].y);
+      ptx::tmem_st_wait();
       ptx::tc_fence_before_sync();
       ptx::mbar_arrive(p_ready(s));
     }
 
-    if (ok) ok = ptx::mbar_wait(o_done, (nt - 1) & 1, p.status, 18);
-    if (ok) {
+    if (ok && n > 0) ok = ptx::mbar_wait(o_done(s), 0, p.status, 18);
+    if (ok && n > 0) {
       ptx::tc_fence_after_sync();
-      // total row sum: exchange the two halves' partial sums (buffer of parity nt is free: last used by tile nt-2)
-      float* xb = xchg + (nt & 1) * 2 * kQ;
-      xb[half * kQ + r] = l_part;
-      ok = pair_sync(pair_bar(quarter), (uint32_t)nt, p.status);
-    }
-    if (ok) {
-      const float* xb = xchg + (nt & 1) * 2 * kQ;
-      const float l_run = l_part + xb[(half ^ 1) * kQ + r];
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       const bool live = q0 + r < p.lq;
       __nv_bfloat16* orow = p.out + (((size_t)batch * p.lq + (live ? q0 + r : 0)) * p.heads + head) * HD;
 #pragma unroll
       for (int c = 0; c < HD / 32; ++c) {
-        if ((c & 1) != half) continue;
         uint32_t o[32];
-        ptx::tmem_ld_32x32(tmem_o + lane_base + c * 32, o);
+        ptx::tmem_ld_32x32(tmem_o(s) + lane_base + c * 32, o);
         ptx::tmem_ld_wait();
         if (live) {
 #pragma unroll
@@ -304,14 +324,14 @@ __global__ void __launch_bounds__(320, 2) swa_fwd_kernel(const __grid_constant__
           }
         }
       }
-      if (live && half == 0)
+      if (live)
         p.lse[((size_t)batch * p.heads + head) * p.lq + q0 + r] =
             l_run > 0.f ? (m_ref * 0.6931471805599453f + __logf(l_run)) : -INFINITY;
     }
   }
   ptx::tc_fence_before_sync();
   __syncthreads();
-  if (warp == 8) ptx::tmem_dealloc(tmem, 256);
+  if (warp == 8) ptx::tmem_dealloc(tmem, 512);
 }
 
 // ------------------------------------------------------------------------------------ host
@@ -364,20 +384,28 @@ std::vector<at::Tensor> swa_fwd(at::Tensor q, at::Tensor k, at::Tensor v, int64_
   p.lq = lq; p.lk = lk; p.heads = h; p.hd = hd;
   p.window = causal ? (int)window : 0;
   p.causal = causal ? 1 : 0;
-  p.scale_log2 = (float)(scale * 1.4426950408889634);
+  // the kernel takes row maxima before it scales, which needs a positive factor: the sign goes to S, and a scale of
+  // zero becomes one that no product of finite values notices (0 * -inf of a masked key would be NaN)
+  const float scale_log2 = (float)(scale * 1.4426950408889634);
+  p.flip = scale_log2 < 0.f ? 1 : 0;
+  p.scale_log2 = scale_log2 == 0.f ? 1e-37f : fabsf(scale_log2);
   p.out = reinterpret_cast<__nv_bfloat16*>(out.data_ptr());
   p.lse = lse.data_ptr<float>();
   p.status = gemm_status(q).data_ptr<int>();
-  dim3 grid((lq + kQ - 1) / kQ, h, b);
+  // One 128-query tile per CTA as long as every tile has an SM of its own; beyond that two, which cost one and a half
+  // times a single one and fetch K and V once.
+  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  p.tiles = (int64_t)((lq + kQ - 1) / kQ) * h * b <= sms ? 1 : 2;
+  dim3 grid((lq + kQ * p.tiles - 1) / (kQ * p.tiles) * h, b);
   auto stream = at::cuda::getCurrentCUDAStream().stream();
-  auto launch = [&](auto kernel) {
-    C10_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem));
-    kernel<<<grid, 320, kAttnSmem, stream>>>(tq, tk, tv, p);
+  auto launch = [&](auto kernel, int smem) {
+    C10_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kernel<<<grid, kThreads, smem, stream>>>(tq, tk, tv, p);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
   };
-  if (hd == 64) launch(swa_fwd_kernel<64>);
-  else if (hd == 96) launch(swa_fwd_kernel<96>);
-  else launch(swa_fwd_kernel<128>);
+  if (hd == 64) launch(swa_fwd_kernel<64>, SwaCfg<64>::kSmem);
+  else if (hd == 96) launch(swa_fwd_kernel<96>, SwaCfg<96>::kSmem);
+  else launch(swa_fwd_kernel<128>, SwaCfg<128>::kSmem);
   count_launch();
   return {out, lse};
 }
