@@ -50,3 +50,28 @@ def test_attention_tile_edges(b, h, lq, lk, hd, window, causal, scale):
             assert float(got.float().abs().max()) < 2e-2, name
         else:
             assert _rel(got, ref_) < 1e-2, (name, _rel(got, ref_))
+
+
+@pytest.mark.parametrize("bsz,e,r,rows,d", [(1, 1, 256, 128, 128), (3, 2, 384, 384, 128), (2, 3, 512, 256, 384)])
+def test_momentum_and_normalisation(bsz, e, r, rows, d):
+    """Values and gradients against the two separate operations, with each output used alone and both together."""
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(r + d)
+    a, z = (torch.randn(bsz, e, r, d, generator=gen, device=DEV) for _ in range(2))
+    m = torch.rand(bsz, 1, 1, 1, generator=gen, device=DEV)
+    gz, gd = torch.randn(a.shape, generator=gen, device=DEV), torch.randn(a.shape, generator=gen, device=DEV).bfloat16()
+    for use_z, use_d in ((True, True), (True, False), (False, True)):
+        res = []
+        for fused in (True, False):
+            t = [x.clone().requires_grad_() for x in (a, z, m)]
+            if fused:
+                zn, dd = ops.momentum_newton_schulz(*t, rows)
+            else:
+                zn = torch.addcmul(t[0], t[1], t[2])
+                dd = ops.newton_schulz(zn.reshape(-1, rows, d)).reshape(a.shape)
+            outs, cots = zip(*([(zn, gz)] * use_z + [(dd, gd)] * use_d))
+            res.append((zn.detach(), dd.detach(), *torch.autograd.grad(outs, t, cots)))
+        assert _rel(res[0][0], res[1][0]) < 1e-6
+        # the orthogonalisation passes the order of the norms' sums (1e-7) through five bf16 iterations
+        for x, y in zip(res[0][1:], res[1][1:]):
+            assert _rel(x, y) < 3e-2

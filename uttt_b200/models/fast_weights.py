@@ -188,7 +188,14 @@ def apply_pool_update(a02: torch.Tensor, a1: torch.Tensor, state: PoolState, m_c
     m02, m1 = state.m02, state.m1
     bsz, e, inter2, d = m02.shape
     z02, z1 = state.z02, state.z1
-    if z02 is not None and m_coeff is not None:
+    momentum = z02 is not None and m_coeff is not None
+    if momentum and use_muon:
+        z02, d02 = ops.momentum_newton_schulz(a02, z02, m_coeff, inter2 // 2, ns_coeffs)
+        z1, d1 = ops.momentum_newton_schulz(a1, z1, m_coeff, d, ns_coeffs)
+        n02, w02 = ops.pool_step(m02, d02, lr_scale, renorm, compute_dtype)
+        n1, w1 = ops.pool_step(m1, d1, lr_scale, renorm, compute_dtype)
+        return PoolState(w02, w1, n02, n1, z02, z1)
+    if momentum:
         a02 = torch.addcmul(a02, z02, m_coeff.to(a02.dtype))
         a1 = torch.addcmul(a1, z1, m_coeff.to(a1.dtype))
         z02, z1 = a02, a1

@@ -88,6 +88,10 @@ at::Tensor ep_pull_dot(at::Tensor local, std::vector<int64_t> peer_ptrs, at::Ten
                        int64_t cap_rows);
 std::vector<at::Tensor> frob_normalize_fwd(at::Tensor g, double eps);
 at::Tensor frob_normalize_bwd(at::Tensor g, at::Tensor sumsq, at::Tensor dx, double eps);
+std::vector<at::Tensor> momentum_normalize_fwd(at::Tensor a, at::Tensor z, at::Tensor m, int64_t matrices, double eps);
+std::vector<at::Tensor> momentum_normalize_bwd(at::Tensor z_new, at::Tensor z, at::Tensor m, at::Tensor sumsq,
+                                               c10::optional<at::Tensor> dz_new, c10::optional<at::Tensor> dx, double eps,
+                                               bool need_dz, bool need_dm);
 bool pool_step_supported(int64_t D);
 std::vector<at::Tensor> pool_step_fwd(at::Tensor m, at::Tensor d, double lr, int64_t mode);
 std::vector<at::Tensor> pool_step_bwd(at::Tensor m, at::Tensor d, c10::optional<at::Tensor> gn,
@@ -169,6 +173,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ep_pull_dot", &ep_pull_dot);
   m.def("frob_normalize_fwd", &frob_normalize_fwd);
   m.def("frob_normalize_bwd", &frob_normalize_bwd);
+  m.def("momentum_normalize_fwd", &momentum_normalize_fwd);
+  m.def("momentum_normalize_bwd", &momentum_normalize_bwd);
   m.def("pool_step_supported", &pool_step_supported);
   m.def("pool_step_fwd", &pool_step_fwd);
   m.def("pool_step_bwd", &pool_step_bwd);

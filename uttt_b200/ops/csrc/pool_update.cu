@@ -391,4 +391,156 @@ at::Tensor frob_normalize_bwd(at::Tensor g, at::Tensor sumsq, at::Tensor dx, dou
   return dg;
 }
 
+// ------------------------------------------------------------------------------------ momentum + Newton-Schulz input
+// z' = a + m[seq] z and X = z' / (|z'|_F + eps) per matrix, and their VJP
+//   g  = dz' + dX / (r + eps) - z' <dX, z'> / (r (r + eps)^2),   r = |z'|_F
+//   da = g,   dz = m g,   dm[seq] = sum over the matrices of the sequence of <g, z>.
+// Bound by memory.  The squares are summed while z' is written, and the VJP forms da, dz and the products for dm from one
+// read of its operands: as separate operations the broadcast multiply-add alone ran at 3.9 TB/s, and the backward paid an
+// addition, a broadcast product and a product with its reduction on top of the normalisation.  Bank of 113 M values:
+// forward 550 -> 350 us, backward 790 us and the reduction for dm -> 490 us.
+__global__ void __launch_bounds__(256) momentum_sumsq_kernel(const float* __restrict__ a, const float* __restrict__ z,
+                                                             const float* __restrict__ m, float* __restrict__ z_out,
+                                                             float* __restrict__ sumsq, long long per_matrix, int per_seq) {
+  const long long b = blockIdx.y;
+  const float mc = m[b / per_seq];
+  const long long off = b * per_matrix, nv = per_matrix >> 2;
+  float acc = 0.f;
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (long long)gridDim.x * blockDim.x) {
+    float x[4], y[4];
+    load4(a + off + v * 4, x);
+    load4(z + off + v * 4, y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[i] = fmaf(mc, y[i], x[i]);
+      acc = fmaf(x[i], x[i], acc);
+    }
+    store4(z_out + off + v * 4, x);
+  }
+  acc = warp_sum(acc);
+  __shared__ float red[8];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.f;
+    for (int i = 0; i < 8; ++i) s += red[i];
+    atomicAdd(sumsq + b, s);
+  }
+}
+
+// dx, dz_new, dz and dm may be absent; dm[b] collects <g, z> of matrix b
+__global__ void __launch_bounds__(256) momentum_bwd_kernel(const float* __restrict__ z_new, const float* __restrict__ z,
+                                                           const float* __restrict__ m, const __nv_bfloat16* __restrict__ dx,
+                                                           const float* __restrict__ dz_new, const float* __restrict__ sumsq,
+                                                           const float* __restrict__ dot, float eps, float* __restrict__ da,
+                                                           float* __restrict__ dz, float* __restrict__ dm,
+                                                           long long per_matrix, int per_seq) {
+  const long long b = blockIdx.y;
+  const float mc = m[b / per_seq];
+  float inv = 0.f, coef = 0.f;
+  if (dx != nullptr) {
+    const float r = sqrtf(sumsq[b]);
+    inv = 1.f / (r + eps);
+    coef = r > 0.f ? dot[b] * inv * inv / r : 0.f;
+  }
+  const long long off = b * per_matrix, nv = per_matrix >> 2;
+  float acc = 0.f;
+  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (long long)gridDim.x * blockDim.x) {
+    const long long at = off + v * 4;
+    float g[4] = {0.f, 0.f, 0.f, 0.f};
+    if (dz_new != nullptr) load4(dz_new + at, g);
+    if (dx != nullptr) {
+      float d[4], x[4];
+      load4(dx + at, d);
+      load4(z_new + at, x);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[i] += d[i] * inv - x[i] * coef;
+    }
+    store4(da + at, g);
+    if (dm != nullptr) {
+      float y[4];
+      load4(z + at, y);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc = fmaf(g[i], y[i], acc);
+    }
+    if (dz != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[i] *= mc;
+      store4(dz + at, g);
+    }
+  }
+  if (dm == nullptr) return;
+  acc = warp_sum(acc);
+  __shared__ float red[8];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.f;
+    for (int i = 0; i < 8; ++i) s += red[i];
+    atomicAdd(dm + b, s);
+  }
+}
+
+static void check_bank(const at::Tensor& t, int64_t matrices) {
+  TORCH_CHECK(t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() % (4 * matrices) == 0 &&
+              ((uintptr_t)t.data_ptr() & 15) == 0);
+}
+
+// a, z fp32 [S, ...] holding `matrices` equal matrices, m fp32 [S] -> (z' like a, X bf16 like a, sumsq [matrices])
+std::vector<at::Tensor> momentum_normalize_fwd(at::Tensor a, at::Tensor z, at::Tensor m, int64_t matrices, double eps) {
+  c10::cuda::CUDAGuard guard(a.device());
+  check_bank(a, matrices);
+  check_bank(z, matrices);
+  TORCH_CHECK(z.numel() == a.numel() && m.scalar_type() == at::kFloat && m.is_contiguous() && m.numel() > 0 &&
+              matrices % m.numel() == 0 && matrices <= 65535);
+  const long long per = a.numel() / matrices;
+  auto z_new = at::empty_like(a);
+  auto x = at::empty(a.sizes(), a.options().dtype(at::kBFloat16));
+  auto sumsq = at::zeros({matrices}, a.options());
+  auto stream = at::cuda::getCurrentCUDAStream().stream();
+  const dim3 grid = frob_grid(per, (int)matrices);
+  momentum_sumsq_kernel<<<grid, 256, 0, stream>>>(a.data_ptr<float>(), z.data_ptr<float>(), m.data_ptr<float>(),
+                                                 z_new.data_ptr<float>(), sumsq.data_ptr<float>(), per,
+                                                 (int)(matrices / m.numel()));
+  frob_scale_kernel<float><<<grid, 256, 0, stream>>>(z_new.data_ptr<float>(), sumsq.data_ptr<float>(), (float)eps,
+                                                     reinterpret_cast<__nv_bfloat16*>(x.data_ptr()), per);
+  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  count_launch(2);
+  return {z_new, x, sumsq};
+}
+
+// -> (da, dz or empty, dm [S] or empty)
+std::vector<at::Tensor> momentum_normalize_bwd(at::Tensor z_new, at::Tensor z, at::Tensor m, at::Tensor sumsq,
+                                               c10::optional<at::Tensor> dz_new, c10::optional<at::Tensor> dx, double eps,
+                                               bool need_dz, bool need_dm) {
+  c10::cuda::CUDAGuard guard(z_new.device());
+  const int64_t matrices = sumsq.numel();
+  const long long per = z_new.numel() / matrices;
+  auto stream = at::cuda::getCurrentCUDAStream().stream();
+  const dim3 grid = frob_grid(per, (int)matrices);
+  at::Tensor gz, gx, dot;
+  if (dz_new.has_value() && dz_new->defined()) gz = dz_new->to(at::kFloat).contiguous();
+  if (dx.has_value() && dx->defined()) {
+    gx = dx->to(at::kBFloat16).contiguous();
+    dot = at::zeros({matrices}, sumsq.options());
+    frob_partial_kernel<float><<<grid, 256, 0, stream>>>(z_new.data_ptr<float>(),
+                                                         reinterpret_cast<const __nv_bfloat16*>(gx.data_ptr()),
+                                                         dot.data_ptr<float>(), per);
+    count_launch();
+  }
+  auto da = at::empty_like(z_new);
+  auto dz = need_dz ? at::empty_like(z) : at::empty({0}, z.options());
+  auto dm = need_dm ? at::zeros({matrices}, m.options()) : at::empty({0}, m.options());
+  momentum_bwd_kernel<<<grid, 256, 0, stream>>>(
+      z_new.data_ptr<float>(), z.data_ptr<float>(), m.data_ptr<float>(),
+      gx.defined() ? reinterpret_cast<const __nv_bfloat16*>(gx.data_ptr()) : nullptr,
+      gz.defined() ? gz.data_ptr<float>() : nullptr, sumsq.data_ptr<float>(), gx.defined() ? dot.data_ptr<float>() : nullptr,
+      (float)eps, da.data_ptr<float>(), need_dz ? dz.data_ptr<float>() : nullptr, need_dm ? dm.data_ptr<float>() : nullptr,
+      per, (int)(matrices / m.numel()));
+  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  count_launch();
+  if (need_dm) dm = dm.view({m.numel(), -1}).sum(1);
+  return {da, dz, dm};
+}
+
 }  // namespace uttt

@@ -1473,6 +1473,50 @@ class _FrobNormalize(torch.autograd.Function):
         return cuda_ext(g).frob_normalize_bwd(g, sumsq, dx, ctx.eps), None
 
 
+class _MomentumNormalize(torch.autograd.Function):
+    """``z' = a + m z`` per sequence and ``x = z' / (|z'|_F + eps)`` (bf16) per matrix, one pass each way over the bank
+    beside the reductions that the norms need."""
+
+    @staticmethod
+    def forward(ctx, a, z, m, matrices, eps):
+        z_new, x, sumsq = cuda_ext(a).momentum_normalize_fwd(a, z, m, int(matrices), float(eps))
+        ctx.save_for_backward(z_new, z, m, sumsq)
+        ctx.eps = float(eps)
+        ctx.set_materialize_grads(False)
+        return z_new, x
+
+    @staticmethod
+    def backward(ctx, dz_new, dx):
+        z_new, z, m, sumsq = ctx.saved_tensors
+        if dz_new is None and dx is None:
+            return None, None, None, None, None
+        _, need_z, need_m = ctx.needs_input_grad[:3]
+        da, dz, dm = cuda_ext(z).momentum_normalize_bwd(z_new, z, m, sumsq, dz_new, dx, ctx.eps, need_z, need_m)
+        return da, dz if need_z else None, dm if need_m else None, None, None
+
+
+def momentum_newton_schulz(a: torch.Tensor, z: torch.Tensor, m: torch.Tensor, rows: int, coeffs=ref.NS5_COEFFS):
+    """Momentum and its orthogonalisation: ``z' = a + m z`` and ``newton_schulz`` of every ``rows``-row matrix of z'.
+
+    a, z: [B, E, R, D] with R a multiple of ``rows``; m: one factor per sequence, shaped to broadcast over them.
+    Returns (z', d) shaped like a; d is bf16 on the kernel path."""
+    bsz, e, r, d = a.shape
+    shape = (bsz * e * (r // rows), rows, d)
+    if _kernel("momentum_normalize_fwd", a) is not None and a.dtype == z.dtype == torch.float32 and a.shape == z.shape \
+            and z.device == a.device and m.device == a.device and m.numel() == bsz and m.shape == (bsz, 1, 1, 1) \
+            and rows % 128 == 0 and d % 128 == 0 and 0 < shape[0] <= 65535:
+        z_new, x = _MomentumNormalize.apply(_aligned(a), _aligned(z), m.reshape(-1).float().contiguous(), shape[0], 1e-7)
+        return z_new, _ns_iterations(x.view(shape), coeffs).view(a.shape)
+    z_new = torch.addcmul(a, z, m.to(a.dtype))
+    return z_new, newton_schulz(z_new.reshape(shape), coeffs).reshape(a.shape)
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous on a 16-byte boundary (a view at an odd offset is copied)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _NSIteration(torch.autograd.Function):
     """One Newton-Schulz iteration ``X' = a X + B X`` (wide; ``A = X X^T``) or ``X' = a X + X B`` (tall;
     ``A = X^T X``) with ``B = b A + c A A``, and its hand-written backward: six batched GEMMs whose epilogues add the
@@ -1539,7 +1583,12 @@ def _newton_schulz_kernels(g, coeffs):
     else:
         x = g.to(torch.bfloat16)
         x = (x / (x.float().norm(dim=(1, 2), keepdim=True) + 1e-7).to(torch.bfloat16)).contiguous()
-    tall = g.size(1) > g.size(2)
+    return _ns_iterations(x, coeffs)
+
+
+def _ns_iterations(x, coeffs):
+    """The iterations on a normalised bf16 stack."""
+    tall = x.size(1) > x.size(2)
     for a, b, c in coeffs:
         if _ns_iteration_ok(x, tall):
             x = _NSIteration.apply(x, a, b, c, tall)
