@@ -2,6 +2,7 @@
 and largest of their ranges, both sides of every rule that picks a variant."""
 import pytest
 import torch
+import torch.nn.functional as F
 
 from uttt_b200 import ops
 from uttt_b200.ops._ext import load
@@ -75,3 +76,22 @@ def test_momentum_and_normalisation(bsz, e, r, rows, d):
         # the orthogonalisation passes the order of the norms' sums (1e-7) through five bf16 iterations
         for x, y in zip(res[0][1:], res[1][1:]):
             assert _rel(x, y) < 3e-2
+
+
+@pytest.mark.parametrize("d", [4, 512, 516, 1536, 2048])
+@pytest.mark.parametrize("renorm", ["restore", "unit", "none"])
+@pytest.mark.parametrize("rows", [1, 3, 700])
+def test_pool_step_row_widths(d, renorm, rows):
+    """One and four warps to a row."""
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(d + rows)
+    m, dd, gn = (torch.randn(rows, d, generator=gen, device=DEV) for _ in range(3))
+    t = [x.clone().requires_grad_() for x in (m, dd)]
+    n, w = ops.pool_step(*t, 0.3, renorm)
+    x = [v.double().requires_grad_() for v in (m, dd)]
+    u = x[0] + x[1] * 0.3
+    want = {"restore": lambda: u / (u.norm(dim=-1, keepdim=True) + 1e-5) * x[0].norm(dim=-1, keepdim=True),
+            "unit": lambda: F.normalize(u, dim=-1), "none": lambda: u}[renorm]()
+    assert _rel(n, want) < 1e-6 and torch.equal(w, n.bfloat16())
+    for a, b in zip(torch.autograd.grad(n, t, gn), torch.autograd.grad(want, x, gn.double())):
+        assert _rel(a, b) < 1e-5

@@ -10,7 +10,8 @@
 //   restore: s = |m| / (|u| + eps);  g_u = s g - u (g.u) s / ((|u| + eps) |u|);  g_m = g_u + m (g.u) / ((|u| + eps) |m|)
 //   unit   : g_u = g / |u| - u (g.u) / |u|^3;                                     g_m = g_u
 //   g_d = lr g_u
-// One warp per row; the row lives in registers between the reduction and the write.
+// One warp per row of up to 512 elements, four warps beyond; the row lives in registers between the reduction and the
+// write.
 // Reference behaviour: flame/custom_models/uttt_moe/modeling_recurrent_lact.py:754-825 (dense apply) and the
 // row re-normalisation of the view-synthesis blocks.
 #include <ATen/ATen.h>
@@ -22,7 +23,8 @@
 
 namespace uttt {
 
-constexpr int kPoolMaxV = 16;        // float4 pieces per lane: rows of up to 2048 elements
+constexpr int kPoolMaxV = 4;         // float4 pieces per lane
+constexpr int kPoolMaxD = 2048;      // four warps to a row of more than 512 elements, one to a shorter one
 enum PoolRenorm { kRestore = 0, kUnit = 1, kNone = 2 };
 
 template <typename T>
@@ -53,22 +55,53 @@ __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, const fl
   *reinterpret_cast<uint2*>(p) = v;
 }
 
-template <typename TD, int MAXV>
+// Sums of a row held by W warps (W = 4: half of a 256-thread block, with a barrier of its own).  `turn` alternates the
+// exchange buffer from one row to the next, so that one barrier per row is enough.
+template <int W, int N>
+__device__ __forceinline__ void row_sums(float (&v)[N], int& turn) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = warp_sum(v[i]);
+  if constexpr (W > 1) {
+    static_assert(W == 4);
+    __shared__ float part[2][8][N];
+    const int warp = threadIdx.x >> 5, first = warp & ~(W - 1);
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) part[turn][warp][i] = v[i];
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + first / W), "n"(32 * W) : "memory");
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      v[i] = 0.f;
+#pragma unroll
+      for (int w = 0; w < W; ++w) v[i] += part[turn][first + w][i];
+    }
+    turn ^= 1;
+  }
+}
+
+// Bound by memory.  A row of 1536 elements on one warp needs 12 vectors per lane and array in registers (the backward
+// holds three arrays), which left two or three blocks per SM and half the copy rate; on four warps it needs three.
+// 24,576 rows of 1536: forward 113 -> 84 us, backward 252 -> 126 us; 196,608 rows of 384, where the backward no longer
+// reads the master twice: 287 -> 229 us.
+template <typename TD, int W>
 __global__ void __launch_bounds__(256) pool_step_fwd_kernel(const float* __restrict__ m, const TD* __restrict__ d,
                                                             float lr, int mode, float* __restrict__ n_out,
                                                             __nv_bfloat16* __restrict__ w_out, long long rows, int D) {
-  const int lane = threadIdx.x & 31;
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  constexpr int L = 32 * W, MAXV = kPoolMaxV;
+  const int lane = threadIdx.x & (L - 1);
+  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const long long stride = (long long)gridDim.x * blockDim.x / L;
   const int nv = D >> 2;
-  for (long long r = warp; r < rows; r += nwarps) {
+  int turn = 0;
+  for (long long r = first; r < rows; r += stride) {
     const float* mr = m + r * D;
     const TD* dr = d + r * D;
     float u[MAXV][4];
     float su = 0.f, sm = 0.f;
 #pragma unroll
     for (int j = 0; j < MAXV; ++j) {
-      int v = lane + 32 * j;
+      int v = lane + L * j;
       if (v < nv) {
         float a[4], b[4];
         load4(mr + v * 4, a);
@@ -83,13 +116,15 @@ __global__ void __launch_bounds__(256) pool_step_fwd_kernel(const float* __restr
     }
     float s = 1.f;
     if (mode != kNone) {
-      su = warp_sum(su);
-      sm = warp_sum(sm);
+      float t[2] = {su, sm};
+      row_sums<W>(t, turn);
+      su = t[0];
+      sm = t[1];
       s = (mode == kRestore) ? sqrtf(sm) / (sqrtf(su) + 1e-5f) : 1.f / fmaxf(sqrtf(su), 1e-12f);
     }
 #pragma unroll
     for (int j = 0; j < MAXV; ++j) {
-      int v = lane + 32 * j;
+      int v = lane + L * j;
       if (v < nv) {
         float o[4];
 #pragma unroll
@@ -101,27 +136,29 @@ __global__ void __launch_bounds__(256) pool_step_fwd_kernel(const float* __restr
   }
 }
 
-template <typename TD, int MAXV>
+template <typename TD, int W>
 __global__ void __launch_bounds__(256) pool_step_bwd_kernel(const float* __restrict__ m, const TD* __restrict__ d,
                                                             const float* __restrict__ gn,
                                                             const __nv_bfloat16* __restrict__ gw, float lr, int mode,
                                                             float* __restrict__ gm_out, TD* __restrict__ gd_out,
                                                             long long rows, int D) {
-  const int lane = threadIdx.x & 31;
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  constexpr int L = 32 * W, MAXV = kPoolMaxV;
+  const int lane = threadIdx.x & (L - 1);
+  const long long first = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const long long stride = (long long)gridDim.x * blockDim.x / L;
   const int nv = D >> 2;
-  for (long long r = warp; r < rows; r += nwarps) {
+  int turn = 0;
+  for (long long r = first; r < rows; r += stride) {
     const float* mr = m + r * D;
     const TD* dr = d + r * D;
-    float u[MAXV][4], g[MAXV][4];
+    float u[MAXV][4], g[MAXV][4], a[MAXV][4];
     float su = 0.f, sm = 0.f, gu = 0.f;
 #pragma unroll
     for (int j = 0; j < MAXV; ++j) {
-      int v = lane + 32 * j;
+      int v = lane + L * j;
       if (v < nv) {
-        float a[4], b[4];
-        load4(mr + v * 4, a);
+        float b[4];
+        load4(mr + v * 4, a[j]);
         load4(dr + v * 4, b);
 #pragma unroll
         for (int i = 0; i < 4; ++i) g[j][i] = 0.f;
@@ -134,18 +171,20 @@ __global__ void __launch_bounds__(256) pool_step_bwd_kernel(const float* __restr
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          u[j][i] = fmaf(lr, b[i], a[i]);
+          u[j][i] = fmaf(lr, b[i], a[j][i]);
           su = fmaf(u[j][i], u[j][i], su);
-          sm = fmaf(a[i], a[i], sm);
+          sm = fmaf(a[j][i], a[j][i], sm);
           gu = fmaf(g[j][i], u[j][i], gu);
         }
       }
     }
     float cg = 1.f, cu = 0.f, cm = 0.f;      // g_u = cg * g - cu * u ;  g_m = g_u + cm * m
     if (mode != kNone) {
-      su = warp_sum(su);
-      sm = warp_sum(sm);
-      gu = warp_sum(gu);
+      float t[3] = {su, sm, gu};
+      row_sums<W>(t, turn);
+      su = t[0];
+      sm = t[1];
+      gu = t[2];
       const float nu = sqrtf(su), nm = sqrtf(sm);
       if (mode == kRestore) {
         const float den = nu + 1e-5f;
@@ -160,14 +199,13 @@ __global__ void __launch_bounds__(256) pool_step_bwd_kernel(const float* __restr
     }
 #pragma unroll
     for (int j = 0; j < MAXV; ++j) {
-      int v = lane + 32 * j;
+      int v = lane + L * j;
       if (v < nv) {
-        float a[4], o_m[4], o_d[4];
-        if (cm != 0.f) load4(mr + v * 4, a);
+        float o_m[4], o_d[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           float t = cg * g[j][i] - cu * u[j][i];
-          o_m[i] = (cm != 0.f) ? fmaf(cm, a[i], t) : t;
+          o_m[i] = (cm != 0.f) ? fmaf(cm, a[j][i], t) : t;
           o_d[i] = lr * t;
         }
         store4(gm_out + r * D + v * 4, o_m);
@@ -177,13 +215,13 @@ __global__ void __launch_bounds__(256) pool_step_bwd_kernel(const float* __restr
   }
 }
 
-static int pool_blocks(long long rows) {
+static int pool_blocks(long long rows, int rows_per_block) {
   int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  long long want = (rows + 7) / 8;
+  long long want = (rows + rows_per_block - 1) / rows_per_block;
   return (int)std::max<long long>(1, std::min<long long>(want, (long long)sms * 8));
 }
 
-bool pool_step_supported(int64_t D) { return D % 4 == 0 && D <= 128 * kPoolMaxV; }
+bool pool_step_supported(int64_t D) { return D % 4 == 0 && D <= kPoolMaxD; }
 
 // m [.., D] fp32, d same shape (bf16 or fp32) -> (n fp32, w bf16)
 std::vector<at::Tensor> pool_step_fwd(at::Tensor m, at::Tensor d, double lr, int64_t mode) {
@@ -195,15 +233,15 @@ std::vector<at::Tensor> pool_step_fwd(at::Tensor m, at::Tensor d, double lr, int
   auto n = at::empty_like(m);
   auto w = at::empty(m.sizes(), m.options().dtype(at::kBFloat16));
   auto stream = at::cuda::getCurrentCUDAStream().stream();
-  const int blocks = pool_blocks(rows);
+  const int blocks = pool_blocks(rows, D <= 512 ? 8 : 2);
   auto go = [&](auto* dp) {
     using TD = std::remove_cv_t<std::remove_pointer_t<decltype(dp)>>;
     if (D <= 512)
-      pool_step_fwd_kernel<TD, 4><<<blocks, 256, 0, stream>>>(m.data_ptr<float>(), dp, (float)lr, (int)mode,
+      pool_step_fwd_kernel<TD, 1><<<blocks, 256, 0, stream>>>(m.data_ptr<float>(), dp, (float)lr, (int)mode,
                                                               n.data_ptr<float>(),
                                                               reinterpret_cast<__nv_bfloat16*>(w.data_ptr()), rows, D);
     else
-      pool_step_fwd_kernel<TD, kPoolMaxV><<<blocks, 256, 0, stream>>>(
+      pool_step_fwd_kernel<TD, 4><<<blocks, 256, 0, stream>>>(
           m.data_ptr<float>(), dp, (float)lr, (int)mode, n.data_ptr<float>(),
           reinterpret_cast<__nv_bfloat16*>(w.data_ptr()), rows, D);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -235,14 +273,14 @@ std::vector<at::Tensor> pool_step_bwd(at::Tensor m, at::Tensor d, c10::optional<
   auto gm = at::empty_like(m);
   auto gd = at::empty_like(d);
   auto stream = at::cuda::getCurrentCUDAStream().stream();
-  const int blocks = pool_blocks(rows);
+  const int blocks = pool_blocks(rows, D <= 512 ? 8 : 2);
   auto go = [&](auto* dp, auto* gp) {
     using TD = std::remove_cv_t<std::remove_pointer_t<decltype(dp)>>;
     if (D <= 512)
-      pool_step_bwd_kernel<TD, 4><<<blocks, 256, 0, stream>>>(m.data_ptr<float>(), dp, gnp, gwp, (float)lr, (int)mode,
+      pool_step_bwd_kernel<TD, 1><<<blocks, 256, 0, stream>>>(m.data_ptr<float>(), dp, gnp, gwp, (float)lr, (int)mode,
                                                               gm.data_ptr<float>(), gp, rows, D);
     else
-      pool_step_bwd_kernel<TD, kPoolMaxV><<<blocks, 256, 0, stream>>>(m.data_ptr<float>(), dp, gnp, gwp, (float)lr,
+      pool_step_bwd_kernel<TD, 4><<<blocks, 256, 0, stream>>>(m.data_ptr<float>(), dp, gnp, gwp, (float)lr,
                                                                       (int)mode, gm.data_ptr<float>(), gp, rows, D);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
   };
