@@ -19,6 +19,7 @@ from typing import Optional, Tuple
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad as fwAD
 
 from . import reference as ref
 from ._ext import cuda_ext, has
@@ -81,6 +82,26 @@ def _note_fallback(op: str, t, why: str = "") -> None:
                                   f"{' (' + why + ')' if why else ''}; set UTTT_B200_STRICT=0 to run it as plain PyTorch")
 
 
+class _NoGraph:
+    """Stands in for the autograd context of a forward whose backward cannot happen."""
+    needs_input_grad = (False,) * 32
+
+    def save_for_backward(self, *tensors):
+        pass
+
+    mark_non_differentiable = mark_dirty = set_materialize_grads = save_for_backward
+
+
+def _run(fn, *args):
+    """``fn.apply(*args)``; with gradients off, the forward by itself.  Generation, scoring and rendering issue a few
+    hundred small kernels per call and wait for the host: at batch one a decoded token made 206 autograd nodes that were
+    dropped at once.  Function transforms, forward-mode differentiation and tracing look at the node, so they keep it."""
+    if torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or fwAD._current_level >= 0 \
+            or torch._C._get_tracing_state() is not None or torch.compiler.is_compiling():
+        return fn.apply(*args)
+    return fn.forward(_NoGraph(), *args)
+
+
 # =========================================================================== norms
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
@@ -103,7 +124,7 @@ class _RMSNorm(torch.autograd.Function):
 
 def rms_norm(x: torch.Tensor, weight: Optional[torch.Tensor], eps: float = 1e-6) -> torch.Tensor:
     if _kernel("rms_norm_fwd", x) is not None and x.shape[-1] % 8 == 0:
-        return _RMSNorm.apply(x, weight, eps)
+        return _run(_RMSNorm, x, weight, eps)
     _note_fallback("rms_norm", x)
     return ref.rms_norm(x, weight, eps)
 
@@ -134,7 +155,7 @@ class _RMSNormGated(torch.autograd.Function):
 def rms_norm_gated(x: torch.Tensor, weight: Optional[torch.Tensor], gate: torch.Tensor, eps: float = 1e-6):
     """``rms_norm(x, weight) * gate[..., None]`` with one factor per row (``gate.shape == x.shape[:-1]``)."""
     if _kernel("rms_norm_gated_fwd", x) is not None and x.shape[-1] % 8 == 0 and x.shape[-1] <= 4096:
-        return _RMSNormGated.apply(x, weight, gate, eps)
+        return _run(_RMSNormGated, x, weight, gate, eps)
     return rms_norm(x, weight, eps) * gate.unsqueeze(-1).to(x.dtype)
 
 
@@ -169,7 +190,7 @@ class _AddRMSNorm(torch.autograd.Function):
 def add_rms_norm(x: torch.Tensor, delta: torch.Tensor, weight: Optional[torch.Tensor], eps: float = 1e-6):
     """Residual addition fused with the norm that follows it: returns (x + delta, rms_norm(x + delta) * weight)."""
     if _kernel("add_rms_norm_fwd", x) is not None and x.shape[-1] % 8 == 0 and x.shape[-1] <= 4096:
-        return _AddRMSNorm.apply(x, delta, weight, eps)
+        return _run(_AddRMSNorm, x, delta, weight, eps)
     s = x + delta
     return s, ref.rms_norm(s, weight, eps)
 
@@ -203,7 +224,7 @@ def embedding(ids: torch.Tensor, table: torch.Tensor, padding_idx: Optional[int]
     """table[ids] with the gather / scatter-add kernels on a GPU (ids: integer tensor of any shape)."""
     if _kernel("embedding_fwd", table) is not None and ids.is_cuda and table.shape[1] % 8 == 0 \
             and table.dtype in (torch.bfloat16, torch.float32):
-        return _Embedding.apply(ids.long(), table, padding_idx)
+        return _run(_Embedding, ids.long(), table, padding_idx)
     return torch.nn.functional.embedding(ids, table, padding_idx)
 
 
@@ -239,13 +260,13 @@ class _Rope(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         offset, theta, inverse = ctx.args
-        return _Rope.apply(dy, offset, theta, not inverse), None, None, None
+        return _run(_Rope, dy, offset, theta, not inverse), None, None, None
 
 
 def rope(x: torch.Tensor, offset: int, theta: float, inverse: bool = False) -> torch.Tensor:
     """Rotary embedding (first-half/second-half pairing) on x: [b, l, nh, hd]."""
     if _kernel("rope_fwd", x) is not None and x.shape[-1] % 2 == 0:
-        return _Rope.apply(x, offset, theta, inverse)
+        return _run(_Rope, x, offset, theta, inverse)
     _note_fallback("rope", x)
     return ref.rope(x, offset, theta, inverse)
 
@@ -284,7 +305,7 @@ def fw_qk_prep(x, scale, shift, fw_heads: int, rope_dim: int, theta: float, offs
     d = x.shape[-1]
     ok = (d // fw_heads) % 8 == 0 and (rope_dim == 0 or (rope_dim % 2 == 0 and (d // fw_heads) % rope_dim == 0))
     if _kernel("fw_qk_prep_fwd", x) is not None and ok:
-        return _FwQkPrep.apply(x, scale, shift, fw_heads, rope_dim, theta, offset, silu, norm)
+        return _run(_FwQkPrep, x, scale, shift, fw_heads, rope_dim, theta, offset, silu, norm)
     _note_fallback("fw_qk_prep", x)
     return ref.fw_qk_prep(x, scale, shift, fw_heads, rope_dim, theta, offset, silu, norm)
 
@@ -331,7 +352,7 @@ def swa_attention(q, k, v, window: Optional[int], causal: bool = True, scale: Op
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
     if _kernel("swa_fwd", q) is not None and q.dtype == torch.bfloat16 and q.shape[-1] in (64, 96, 128) \
             and q.shape[2] == k.shape[2]:
-        return _SWA.apply(q, k, v, window, causal, scale, reuse if torch.is_grad_enabled() else None)
+        return _run(_SWA, q, k, v, window, causal, scale, reuse if torch.is_grad_enabled() else None)
     if q.is_cuda:
         _note_fallback("swa_attention", q, "head dim or head grouping outside the kernel")
         return _sdpa_attention(q, k, v, window, causal, scale)
@@ -605,7 +626,7 @@ def split_linear(x: torch.Tensor, weight: torch.Tensor, n: int):
     if not x.is_cuda or weight.shape[0] % n != 0:
         y = torch.nn.functional.linear(x, weight)
         return tuple(t.contiguous() for t in y.chunk(n, dim=-1))
-    return _SplitLinear.apply(x, weight, n)
+    return _run(_SplitLinear, x, weight, n)
 
 
 def fanout_linear(x: torch.Tensor, weights, biases=None):
@@ -614,7 +635,7 @@ def fanout_linear(x: torch.Tensor, weights, biases=None):
     biases = [None] * len(weights) if biases is None else list(biases)
     if not x.is_cuda:
         return tuple(torch.nn.functional.linear(x, w, b) for w, b in zip(weights, biases))
-    return _FanoutLinear.apply(x, len(weights), *weights, *biases)
+    return _run(_FanoutLinear, x, len(weights), *weights, *biases)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -672,7 +693,7 @@ def stacked_linear(x: torch.Tensor, wa: torch.Tensor, wb: torch.Tensor) -> torch
     """``cat(x @ W_a^T, x @ W_b^T)`` along the last dim, one GEMM."""
     if not x.is_cuda:
         return torch.nn.functional.linear(x, torch.cat([wa, wb], dim=0))
-    return _StackedLinear.apply(x, wa, wb)
+    return _run(_StackedLinear, x, wa, wb)
 
 
 # =========================================================================== view-synthesis decoder tail
@@ -696,7 +717,7 @@ def patch_decode(y: torch.Tensor, target: Optional[torch.Tensor], views: int, he
     """Decoder logits [B, V*T, P*P*3] -> (sigmoid image [B, V, 3, H, W] fp32, squared error per view [B, V]).
     Channel order inside a token is (ph, pw, c); ``target`` may be None (then the error sums are zero)."""
     if _kernel("patch_decode_fwd", y) is not None and y.dtype in (torch.bfloat16, torch.float32):
-        return _PatchDecode.apply(y, None if target is None else target.float().contiguous(), views, height, width,
+        return _run(_PatchDecode, y, None if target is None else target.float().contiguous(), views, height, width,
                                   patch)
     b = y.shape[0]
     hh, ww = height // patch, width // patch
@@ -735,7 +756,7 @@ def pool_step(m: torch.Tensor, d: torch.Tensor, lr: float, renorm: str = "restor
     ext = _kernel("pool_step_fwd", m)
     if ext is not None and m.dtype == torch.float32 and compute_dtype == torch.bfloat16 \
             and d.dtype in (torch.bfloat16, torch.float32) and ext.pool_step_supported(m.shape[-1]):
-        return _PoolStep.apply(m, d, lr, _POOL_MODES[renorm])
+        return _run(_PoolStep, m, d, lr, _POOL_MODES[renorm])
     n = m + d.float() * lr
     if renorm == "restore":
         n = n / (n.norm(dim=-1, keepdim=True) + 1e-5) * m.norm(dim=-1, keepdim=True)
@@ -798,7 +819,7 @@ def route_topk(rows, router, bias, topk: int, alpha: float = 1.0, bias_in_logits
     rscale = router_scale if router_scale > 0 else math.sqrt(float(e))
     ext = _kernel("router_fwd", rows)
     if ext is not None and ext.router_supported(d, e, topk) and rows.dtype in (torch.bfloat16, torch.float32):
-        idx, w, psum = _Router.apply(rows.reshape(bsz * n, d).contiguous(), router.float().contiguous(),
+        idx, w, psum = _run(_Router, rows.reshape(bsz * n, d).contiguous(), router.float().contiguous(),
                                      None if bias is None else bias.detach(), topk, n, alpha, bias_in_logits, renorm,
                                      _ROUTER_MODES[router_type], rscale, norm_eps,
                                      reuse if torch.is_grad_enabled() else None)
@@ -842,7 +863,7 @@ class _Permute(torch.autograd.Function):
     def backward(ctx, dout):
         dest, weights, x, offsets, sizes = ctx.saved_tensors
         if weights is None:
-            return _Unpermute.apply(dout, dest, None, offsets, sizes), None, None, None, None, None
+            return _run(_Unpermute, dout, dest, None, offsets, sizes), None, None, None, None, None
         ext = cuda_ext(dout)
         dout = dout.contiguous()
         dx = ext.unpermute_rows(dout, dest, weights)
@@ -864,7 +885,7 @@ class _Unpermute(torch.autograd.Function):
     def backward(ctx, dout):
         y, dest, weights, offsets, sizes = ctx.saved_tensors
         if weights is None:
-            return _Permute.apply(dout, dest, ctx.rows, None, offsets, sizes), None, None, None, None
+            return _run(_Permute, dout, dest, ctx.rows, None, offsets, sizes), None, None, None, None
         ext = cuda_ext(y)
         dy, dw = ext.unpermute_rows_bwd(dout.contiguous(), y, dest, weights, offsets, sizes)
         return dy, None, dw.to(weights.dtype), None, None
@@ -874,7 +895,7 @@ def permute_rows(x: torch.Tensor, plan: GroupPlan, weights: Optional[torch.Tenso
     """[R, D] token-major rows -> [rows_padded, D] expert-major (each row copied to its top-k groups,
     copy j scaled by ``weights[i, j]`` when given)."""
     if _kernel("permute_rows", x) is not None and x.shape[-1] % 8 == 0:
-        return _Permute.apply(x, plan.dest, plan.rows_padded, weights, plan.offsets, plan.sizes)
+        return _run(_Permute, x, plan.dest, plan.rows_padded, weights, plan.offsets, plan.sizes)
     if weights is None:
         _note_fallback("permute_rows", x)
         return ref.permute_rows(x, plan.dest, plan.rows_padded)
@@ -887,7 +908,7 @@ def permute_rows(x: torch.Tensor, plan: GroupPlan, weights: Optional[torch.Tenso
 def unpermute_rows(y: torch.Tensor, plan: GroupPlan, weights: Optional[torch.Tensor]) -> torch.Tensor:
     """Expert-major rows back to token-major, summing the top-k copies with ``weights`` [R, k]."""
     if _kernel("unpermute_rows", y) is not None and y.shape[-1] % 8 == 0:
-        return _Unpermute.apply(y, plan.dest, weights, plan.offsets, plan.sizes)
+        return _run(_Unpermute, y, plan.dest, weights, plan.offsets, plan.sizes)
     _note_fallback("unpermute_rows", y)
     return ref.unpermute_rows(y, plan.dest, weights)
 
@@ -1050,7 +1071,7 @@ class _GGTN(torch.autograd.Function):
 def gg_nt(x, w, plan: GroupPlan):
     """out[r] = x[r] @ w[group(r)]^T;  x [R, K], w [G, N, K] -> [R, N]."""
     if _gg_kernel_ok(x, w) and _gg_dims_ok(x.shape[1], w.shape[1]):
-        return _GGNT.apply(x, w, plan)
+        return _run(_GGNT, x, w, plan)
     _note_fallback("gg_nt", x)
     return ref.gg_nt(x, w, plan.tile_group)
 
@@ -1058,7 +1079,7 @@ def gg_nt(x, w, plan: GroupPlan):
 def gg_nn(x, w, plan: GroupPlan):
     """out[r] = x[r] @ w[group(r)];  x [R, K], w [G, K, N] -> [R, N]."""
     if _gg_kernel_ok(x, w) and _gg_dims_ok(x.shape[1], w.shape[2]):
-        return _GGNN.apply(x, w, plan)
+        return _run(_GGNN, x, w, plan)
     _note_fallback("gg_nn", x)
     return ref.gg_nn(x, w, plan.tile_group)
 
@@ -1066,10 +1087,10 @@ def gg_nn(x, w, plan: GroupPlan):
 def gg_tn(a, b, plan: GroupPlan, out_dtype: torch.dtype = torch.float32):
     """out[g] = sum_{r in group g} a[r]^T b[r];  a [R, M], b [R, N] -> [G, M, N] (fp32 accumulation)."""
     if _gg_kernel_ok(a, b) and a.shape[1] % 128 == 0 and b.shape[1] % 64 == 0:
-        return _GGTN.apply(a, b, plan, out_dtype)
+        return _run(_GGTN, a, b, plan, out_dtype)
     if _gg_kernel_ok(a, b) and b.shape[1] % 128 == 0 and a.shape[1] % 64 == 0:
         # the kernel wants 128 rows of output per tile: compute the transposed product and view it back
-        return _GGTN.apply(b, a, plan, out_dtype).transpose(1, 2)
+        return _run(_GGTN, b, a, plan, out_dtype).transpose(1, 2)
     _note_fallback("gg_tn", a)
     return ref.gg_tn(a, b, plan.tile_group, plan.num_groups, out_dtype)
 
@@ -1104,7 +1125,7 @@ class _SwiGLUBwd(torch.autograd.Function):
 
 def swiglu(y02: torch.Tensor) -> torch.Tensor:
     if _kernel("swiglu_fwd", y02) is not None and y02.shape[-1] % 16 == 0:
-        return _SwiGLU.apply(y02)
+        return _run(_SwiGLU, y02)
     _note_fallback("swiglu", y02)
     return ref.swiglu(y02)
 
@@ -1153,7 +1174,7 @@ def _gg_swiglu_ok(x, w02) -> bool:
 def gg_swiglu(x, w02, plan: GroupPlan):
     """Grouped SwiGLU hidden activation: x [R, K], w02 [G, 2I, K] (gate rows, then up rows) -> [R, I]."""
     if _gg_swiglu_ok(x, w02):
-        return _GGSwiGLU.apply(x, w02, plan)
+        return _run(_GGSwiGLU, x, w02, plan)
     return swiglu(gg_nt(x, w02, plan))
 
 
