@@ -5,6 +5,7 @@ import torch
 import torch.nn.functional as F
 
 from uttt_b200 import ops
+from uttt_b200.ops import reference as ref
 from uttt_b200.ops._ext import load
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +96,67 @@ def test_pool_step_row_widths(d, renorm, rows):
     assert _rel(n, want) < 1e-6 and torch.equal(w, n.bfloat16())
     for a, b in zip(torch.autograd.grad(n, t, gn), torch.autograd.grad(want, x, gn.double())):
         assert _rel(a, b) < 1e-5
+
+
+# Rows of 1 to 33 and more 16-byte vectors: every lane-group width and the remainders on both sides, row counts that leave
+# groups of the last warp without a row.
+@pytest.mark.parametrize("d", [8, 32, 40, 64, 72, 128, 136, 192, 256, 264, 384])
+@pytest.mark.parametrize("rows", [1, 7, 1001])
+def test_row_kernels_lane_groups(d, rows):
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(d + rows)
+    x, g, delta = (torch.randn(rows, d, generator=gen, device=DEV) for _ in range(3))
+    weight, gate = torch.rand(d, generator=gen, device=DEV) + 0.5, torch.rand(rows, generator=gen, device=DEV)
+    leaves = [t.clone().requires_grad_() for t in (x, weight, gate, delta)]
+    exact = [t.double().requires_grad_() for t in (x, weight, gate, delta)]
+
+    def norm(t, w):
+        return t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + 1e-5) * w
+
+    y = ops.rms_norm(leaves[0], leaves[1], 1e-5) + ops.rms_norm_gated(leaves[0], leaves[1], leaves[2], 1e-5)
+    s, z = ops.add_rms_norm(leaves[0], leaves[3], leaves[1], 1e-5)
+    want = norm(exact[0], exact[1]) * (1 + exact[2][:, None])
+    ws = exact[0] + exact[3]
+    got = torch.autograd.grad([y, s, z], leaves, [g, g, g])
+    expect = torch.autograd.grad([want, ws, norm(ws, exact[1])], exact, [g.double()] * 3)
+    for a, b in zip((y, s, z, *got), (want, ws, norm(ws, exact[1]), *expect)):
+        assert _rel(a, b) < 1e-5                                 # fp32 throughout
+    # scatter into the padded layout and back
+    plan = ops.build_group_plan(torch.randint(0, 3, (1, rows, 2), generator=gen, device=DEV), 3)
+    wts = torch.rand(rows, 2, generator=gen, device=DEV).requires_grad_()
+    xp = ops.permute_rows(leaves[0], plan)
+    back = ops.unpermute_rows(xp, plan, wts)
+    dx, dw = torch.autograd.grad(back, [leaves[0], wts], g)
+    total = wts.detach().sum(1, keepdim=True)
+    assert _rel(back, x * total) < 1e-6 and _rel(dx, g * total) < 1e-6
+    assert _rel(dw, (x * g).sum(1, keepdim=True).expand(-1, 2)) < 1e-4
+
+
+@pytest.mark.parametrize("heads,head,rope", [(8, 16, 0), (3, 64, 0), (8, 64, 32), (2, 192, 64), (4, 192, 192), (1, 512, 0), (1, 1024, 128)])
+@pytest.mark.parametrize("rows", [1, 37])
+def test_qk_prep_lane_groups(heads, head, rope, rows):
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(heads * head + rows)
+    x, g = (torch.randn(2, rows, heads * head, generator=gen, device=DEV) for _ in range(2))
+    scale, shift = torch.rand(heads * head, generator=gen, device=DEV) + 0.5, torch.randn(heads * head, generator=gen, device=DEV) * 0.1
+    for affine in (True, False):
+        mine = [t.clone().requires_grad_() for t in (x, scale, shift)]
+        theirs = [t.clone().requires_grad_() for t in (x, scale, shift)]
+        run = [(fn(t[0], t[1] if affine else None, t[2] if affine else None, heads, rope, 1e4, 5, True, "l2"), t)
+               for fn, t in ((ops.fw_qk_prep, mine), (ref.fw_qk_prep, theirs))]
+        assert _rel(run[0][0], run[1][0]) < 1e-5
+        grads = [torch.autograd.grad(y, t if affine else t[:1], g) for y, t in run]
+        for a, b in zip(*grads):
+            assert _rel(a, b) < 1e-4                             # sums over all rows, fast exponentials
+
+
+@pytest.mark.parametrize("bsz,n,e,k", [(1, 1, 1, 1), (5, 300, 256, 2), (2, 9000, 64, 1), (1, 20000, 16, 2)])
+def test_group_plan_scan(bsz, n, e, k):
+    """More groups than the scan's block has threads, and more blocks of entries than it fetches at a time."""
+    load(required=True)
+    idx = torch.randint(0, e, (bsz, n, k), generator=torch.Generator().manual_seed(n)).to(DEV)
+    plan = ops.build_group_plan(idx, e)
+    dest, offsets, sizes, tile_group, rows = ref.build_group_plan(idx, e)
+    for a, b in ((plan.dest, dest), (plan.offsets, offsets), (plan.sizes, sizes), (plan.tile_group, tile_group)):
+        assert torch.equal(a.cpu().long(), b.cpu().long())
+    assert plan.rows_padded == rows

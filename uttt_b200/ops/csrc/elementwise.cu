@@ -34,24 +34,85 @@ template <typename T> static inline const T* optr(const c10::optional<at::Tensor
 static inline cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 static inline int sm_count() { return at::cuda::getCurrentDeviceProperties()->multiProcessorCount; }
 
+// ------------------------------------------------------------------------------------ lane groups
+// Row kernels give a row to G consecutive lanes, G = the power of two that covers the row's 16-byte vectors (32 when
+// there are more), so that a warp works on 32 / G narrow rows at once: a head of 64 elements has 8 vectors, and one
+// such row per warp leaves three lanes of four idle and a quarter of the bytes in flight.  The row loops are
+// warp-uniform (a group past the end repeats the last row and stores nothing), so the shuffles see full warps.
+// Heads of 64, 24,576 x 8 rows: memory preprocessing 20 -> 9 us forward, 48 -> 13 us backward.  Heads of 192, 2048 x 4
+// rows: 22 -> 20 us backward.
+template <int G>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// the same value of every group of the warp, summed over the groups
+template <int G>
+__device__ __forceinline__ float across_groups(float v) {
+#pragma unroll
+  for (int o = 16; o >= G; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <typename F>
+static inline void with_lanes(int vectors, F&& f) {
+  if (vectors <= 4) f(std::integral_constant<int, 4>{});
+  else if (vectors <= 8) f(std::integral_constant<int, 8>{});
+  else if (vectors <= 16) f(std::integral_constant<int, 16>{});
+  else f(std::integral_constant<int, 32>{});
+}
+
+// out[c] = sum over p of partial[p, c]: the per-block partial sums of a kernel.  32 columns per block, 32 row strands
+// each, so that a few hundred partial rows are a handful of loads in flight per thread: 3.7 us for 592 x 768, where the
+// general reduction took 11.
+__global__ void __launch_bounds__(1024) col_sum_kernel(const float* __restrict__ partial, float* __restrict__ out, int rows,
+                                                       long long cols) {
+  __shared__ float part[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long long c = (long long)blockIdx.x * 32 + tx;
+  float acc = 0.f;
+  if (c < cols) {
+#pragma unroll 4
+    for (int r = ty; r < rows; r += 32) acc += partial[(size_t)r * cols + c];
+  }
+  part[ty][tx] = acc;
+  __syncthreads();
+  const float v = warp_sum(part[tx][ty]);
+  const long long co = (long long)blockIdx.x * 32 + ty;
+  if (tx == 0 && co < cols) out[co] = v;
+}
+at::Tensor col_sum(at::Tensor partial) {
+  const long long cols = partial.numel() / partial.size(0);
+  auto out = at::empty(partial.sizes().slice(1), partial.options());
+  col_sum_kernel<<<(int)((cols + 31) / 32), 1024, 0, at::cuda::getCurrentCUDAStream().stream()>>>(
+      partial.data_ptr<float>(), out.data_ptr<float>(), (int)partial.size(0), cols);
+  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  count_launch();
+  return out;
+}
+
 // ------------------------------------------------------------------------------------ RMSNorm
 // With `add` the kernel first forms the residual sum s = x + add (rounded to T, as the separate addition
 // would), writes it to `sum_out` and normalises s: residual addition and the following norm in one pass.
-template <typename T>
+template <typename T, int G>
 __global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
                                     float* __restrict__ rstd, int rows, int d, float eps,
                                     const T* __restrict__ add = nullptr, T* __restrict__ sum_out = nullptr,
                                     const T* __restrict__ row_scale = nullptr) {
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  int nwarps = (gridDim.x * blockDim.x) >> 5;
-  int nv = d >> 3;
-  for (int r = warp; r < rows; r += nwarps) {
+  constexpr int kRows = 32 / G;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & (G - 1);
+  const int sub = (threadIdx.x & 31) / G;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int nv = d >> 3;
+  for (long long r0 = (long long)warp * kRows; r0 < rows; r0 += (long long)nwarps * kRows) {
+    const bool live = r0 + sub < rows;
+    const int r = live ? (int)r0 + sub : rows - 1;
     const T* xr = x + (size_t)r * d;
     float ss = 0.f;
     if (add != nullptr) {
       const T* ar = add + (size_t)r * d;
       T* sr = sum_out + (size_t)r * d;
-      for (int v = lane; v < nv; v += 32) {
+      for (int v = lane; v < nv; v += G) {
         float f[8], a[8];
         Vec8<T>::load(xr + v * 8, f);
         Vec8<T>::load(ar + v * 8, a);
@@ -60,24 +121,25 @@ __global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict
           f[i] = static_cast<float>(static_cast<T>(f[i] + a[i]));
           ss += f[i] * f[i];
         }
-        Vec8<T>::store(sr + v * 8, f);
+        if (live) Vec8<T>::store(sr + v * 8, f);
       }
-      xr = sr;                                   // the second pass re-reads what this lane just wrote
+      if (live) xr = sr;                         // the second pass re-reads what this lane just wrote
     } else {
-      for (int v = lane; v < nv; v += 32) {
+      for (int v = lane; v < nv; v += G) {
         float f[8];
         Vec8<T>::load(xr + v * 8, f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) ss += f[i] * f[i];
       }
     }
-    ss = warp_sum(ss);
+    ss = group_sum<G>(ss);
     float rs = rsqrtf(ss / d + eps);
+    if (!live) continue;                         // no shuffles below
     if (lane == 0) rstd[r] = rs;
     // an optional per-row factor (the gate of the memory read) is applied to the normalised row in the same pass
     const float rscale = row_scale != nullptr ? rs * to_f<T>(row_scale[r]) : rs;
     T* yr = y + (size_t)r * d;
-    for (int v = lane; v < nv; v += 32) {
+    for (int v = lane; v < nv; v += G) {
       float f[8], g[8];
       Vec8<T>::load(xr + v * 8, f);
       if (w) {
@@ -93,22 +155,26 @@ __global__ void rms_norm_fwd_kernel(const T* __restrict__ x, const T* __restrict
   }
 }
 
-// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)); dw += dy * xhat.  A lane owns vectors lane, lane+32, ...
-// so it can keep its dw columns in registers across rows (d <= 8*32*MAXV).
-template <typename T, int MAXV>
+// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)); dw += dy * xhat.  A lane owns vectors lane, lane+G, ...
+// so it can keep its dw columns in registers across rows (d <= 8*G*MAXV).
+template <typename T, int MAXV, int G>
 __global__ void rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                                     const float* __restrict__ rstd, T* __restrict__ dx, float* __restrict__ dw,
                                     int rows, int d, const T* __restrict__ dres = nullptr,
                                     const T* __restrict__ row_scale = nullptr, float* __restrict__ dscale = nullptr) {
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  int nwarps = (gridDim.x * blockDim.x) >> 5;
-  int nv = d >> 3;
+  constexpr int kRows = 32 / G;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & (G - 1);
+  const int sub = (threadIdx.x & 31) / G;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int nv = d >> 3;
   float acc[MAXV][8];
 #pragma unroll
   for (int j = 0; j < MAXV; ++j)
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
-  for (int r = warp; r < rows; r += nwarps) {
+  for (long long r0 = (long long)warp * kRows; r0 < rows; r0 += (long long)nwarps * kRows) {
+    const bool live = r0 + sub < rows;
+    const int r = live ? (int)r0 + sub : rows - 1;
     const T* xr = x + (size_t)r * d;
     const T* gr = dy + (size_t)r * d;
     float rs = rstd[r];
@@ -117,7 +183,7 @@ __global__ void rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restric
     float dot = 0.f;
 #pragma unroll
     for (int j = 0; j < MAXV; ++j) {
-      int v = lane + 32 * j;
+      int v = lane + G * j;
       if (v < nv) {
         float fx[8], fg[8], fw[8];
         Vec8<T>::load(xr + v * 8, fx);
@@ -128,17 +194,18 @@ __global__ void rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restric
           float xh = fx[i] * rs;
           float gw = w ? fg[i] * fw[i] : fg[i];
           dot += gw * xh;
-          acc[j][i] += fg[i] * sc * xh;
+          if (live) acc[j][i] += fg[i] * sc * xh;
         }
       }
     }
-    dot = warp_sum(dot);
+    dot = group_sum<G>(dot);
+    if (!live) continue;                         // no shuffles below
     if (dscale != nullptr && lane == 0) dscale[r] = dot;
     dot = dot * sc / d;
     T* dxr = dx + (size_t)r * d;
 #pragma unroll
     for (int j = 0; j < MAXV; ++j) {
-      int v = lane + 32 * j;
+      int v = lane + G * j;
       if (v < nv) {
         float fx[8], fg[8], fw[8], o[8];
         Vec8<T>::load(xr + v * 8, fx);
@@ -162,12 +229,18 @@ __global__ void rms_norm_bwd_kernel(const T* __restrict__ dy, const T* __restric
   if (dw) {
     // per-CTA partial sums: the 4 warps of the CTA take turns adding into dw_partial[blockIdx.x, :]
     float* dst = dw + (size_t)blockIdx.x * d;
+    if (G < 32) {
+#pragma unroll
+      for (int j = 0; j < MAXV; ++j)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[j][i] = across_groups<G>(acc[j][i]);
+    }
     int wid = threadIdx.x >> 5;
     for (int turn = 0; turn < (int)(blockDim.x >> 5); ++turn) {
-      if (wid == turn) {
+      if (wid == turn && sub == 0) {
 #pragma unroll
         for (int j = 0; j < MAXV; ++j) {
-          int v = lane + 32 * j;
+          int v = lane + G * j;
           if (v < nv) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -198,17 +271,20 @@ static std::vector<at::Tensor> rms_norm_fwd_impl(at::Tensor x, c10::optional<at:
   auto rstd = at::empty({rows}, x.options().dtype(at::kFloat));
   at::Tensor wc;
   if (w.has_value() && w->defined()) wc = w->to(x.scalar_type()).contiguous();
-  int blocks = std::min((rows + 7) / 8, sm_count() * 8);
   at::Tensor sc;
   if (row_scale.has_value() && row_scale->defined()) {
     sc = row_scale->to(x.scalar_type()).contiguous();
     TORCH_CHECK(sc.numel() == rows, "one factor per row");
   }
   UTTT_DISPATCH_FLOAT(x, {
-    rms_norm_fwd_kernel<T><<<std::max(blocks, 1), 256, 0, cur_stream()>>>(
-        ptr<T>(x), wc.defined() ? ptr<T>(wc) : nullptr, ptr<T>(y), ptr<float>(rstd), rows, d, (float)eps,
-        addc.defined() ? ptr<T>(addc) : nullptr, addc.defined() ? ptr<T>(sum) : nullptr,
-        sc.defined() ? ptr<T>(sc) : nullptr);
+    with_lanes(d / 8, [&](auto lanes) {
+      constexpr int G = decltype(lanes)::value, per_block = 8 * (32 / G);
+      const int blocks = std::max(1, std::min((rows + per_block - 1) / per_block, sm_count() * 8));
+      rms_norm_fwd_kernel<T, G><<<blocks, 256, 0, cur_stream()>>>(
+          ptr<T>(x), wc.defined() ? ptr<T>(wc) : nullptr, ptr<T>(y), ptr<float>(rstd), rows, d, (float)eps,
+          addc.defined() ? ptr<T>(addc) : nullptr, addc.defined() ? ptr<T>(sum) : nullptr,
+          sc.defined() ? ptr<T>(sc) : nullptr);
+    });
   });
   count_launch();
   if (addc.defined()) return {sum, y, rstd};
@@ -239,14 +315,15 @@ static std::vector<at::Tensor> rms_norm_bwd_impl(at::Tensor dy, at::Tensor x, c1
   TORCH_CHECK(d % 8 == 0 && d <= 8 * 32 * 16, "rms_norm_bwd: hidden size must be a multiple of 8 and <= 4096");
   auto dx = at::empty_like(x);
   at::Tensor wc, dw;
-  int blocks = std::max(1, std::min((rows + 3) / 4, sm_count() * 4));
+  const int nv = d / 8;
+  const int per_block = 4 * (nv <= 4 ? 8 : nv <= 8 ? 4 : nv <= 16 ? 2 : 1);      // 4 warps, 32 / G rows each
+  int blocks = std::max(1, std::min((rows + per_block - 1) / per_block, sm_count() * 4));
   if (w.has_value() && w->defined()) {
     wc = w->to(x.scalar_type()).contiguous();
     dw = at::empty({blocks, d}, x.options().dtype(at::kFloat));
   } else {
     dw = at::zeros({1}, x.options().dtype(at::kFloat));
   }
-  int nv = d / 8;
   at::Tensor sc, dsc;
   if (row_scale.has_value() && row_scale->defined()) {
     sc = row_scale->to(x.scalar_type()).contiguous();
@@ -259,18 +336,17 @@ static std::vector<at::Tensor> rms_norm_bwd_impl(at::Tensor dy, at::Tensor x, c1
     const T* rp = dresc.defined() ? ptr<T>(dresc) : nullptr;
     const T* sp = sc.defined() ? ptr<T>(sc) : nullptr;
     float* dsp = sc.defined() ? ptr<float>(dsc) : nullptr;
-    if (nv <= 32 * 2)
-      rms_norm_bwd_kernel<T, 2><<<blocks, 128, 0, cur_stream()>>>(ptr<T>(dy), ptr<T>(x), wp, ptr<float>(rstd),
-                                                                   ptr<T>(dx), dwp, rows, d, rp, sp, dsp);
-    else if (nv <= 32 * 8)
-      rms_norm_bwd_kernel<T, 8><<<blocks, 128, 0, cur_stream()>>>(ptr<T>(dy), ptr<T>(x), wp, ptr<float>(rstd),
-                                                                   ptr<T>(dx), dwp, rows, d, rp, sp, dsp);
-    else
-      rms_norm_bwd_kernel<T, 16><<<blocks, 128, 0, cur_stream()>>>(ptr<T>(dy), ptr<T>(x), wp, ptr<float>(rstd),
-                                                                    ptr<T>(dx), dwp, rows, d, rp, sp, dsp);
+    auto go = [&](auto kernel) {
+      kernel<<<blocks, 128, 0, cur_stream()>>>(ptr<T>(dy), ptr<T>(x), wp, ptr<float>(rstd), ptr<T>(dx), dwp, rows, d, rp, sp,
+                                               dsp);
+    };
+    if (nv <= 32) with_lanes(nv, [&](auto lanes) { go(rms_norm_bwd_kernel<T, 1, decltype(lanes)::value>); });
+    else if (nv <= 32 * 2) go(rms_norm_bwd_kernel<T, 2, 32>);
+    else if (nv <= 32 * 8) go(rms_norm_bwd_kernel<T, 8, 32>);
+    else go(rms_norm_bwd_kernel<T, 16, 32>);
   });
   count_launch();
-  if (wc.defined()) dw = dw.sum(0);
+  if (wc.defined()) dw = col_sum(dw);
   if (sc.defined()) return {dx, dw, dsc};
   return {dx, dw};
 }
@@ -511,8 +587,8 @@ __global__ void fw_qk_prep_bwd_kernel(const T* __restrict__ dy, const T* __restr
   }
 }
 
-// Warp-per-(row, head) forms of the two kernels above, used when a head is at most 64 * MAXP 16-byte vectors wide
-// and half a rotary sub-head is a multiple of 8 elements.  A lane owns pairs of vectors that are half a sub-head
+// Lane-group-per-(row, head) forms of the two kernels above, used when a head is at most 64 * MAXP 16-byte vectors wide
+// and half a rotary sub-head is a multiple of 8 elements.  G lanes hold a head (see "lane groups").  A lane owns pairs of vectors that are half a sub-head
 // apart, i.e. both members of eight rotary pairs: every access is a 16-byte vector, the head's values stay in
 // registers, the rotation needs no exchange, and the forward has no shared memory or block barrier.
 struct QkPairMap {
@@ -526,29 +602,31 @@ struct QkPairMap {
   __device__ __forceinline__ int first_vec(int p) const { return (p / px) * vps + (p % px); }
 };
 
-template <typename T, int MAXP>
+template <typename T, int MAXP, int G>
 __global__ void __launch_bounds__(256) fw_qk_prep_fwd_warp_kernel(
     const T* __restrict__ x, const T* __restrict__ scale, const T* __restrict__ shift,
     const float2* __restrict__ table, T* __restrict__ y, float* __restrict__ inv_out, size_t rows, int d, int heads,
     int rope_dim, int offset, int l, int silu, int norm) {
   const int D = d / heads;
   const QkPairMap map(D, rope_dim);
-  const int lane = threadIdx.x & 31;
-  const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
+  constexpr int kUnits = 32 / G;
+  const int lane = threadIdx.x & (G - 1), sub = (threadIdx.x & 31) / G;
+  const size_t first = (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kUnits;
+  const size_t stride = (((size_t)gridDim.x * blockDim.x) >> 5) * kUnits;
   const size_t units = rows * (size_t)heads;
   const int half = rope_dim >> 1;
   int v0s[MAXP], toff[MAXP];                      // per lane: first vector of each owned pair, its table offset
 #pragma unroll
   for (int j = 0; j < MAXP; ++j) {
-    const int p = lane + 32 * j;
+    const int p = lane + G * j;
     v0s[j] = p < map.npairs ? map.first_vec(p) : -1;
     toff[j] = (p % map.px) * 8;
   }
   // the next unit's values are requested before this unit's arithmetic and reduction, so that a warp always has
   // loads in flight
   float nx[MAXP][2][8];
-  auto fetch = [&](size_t uu) {
+  auto fetch = [&](size_t u0) {
+    const size_t uu = min(u0 + sub, units - 1);
     const size_t r = uu / heads;
     const size_t b = r * d + (uu - r * heads) * (size_t)D;
 #pragma unroll
@@ -558,8 +636,10 @@ __global__ void __launch_bounds__(256) fw_qk_prep_fwd_warp_kernel(
         for (int m = 0; m < 2; ++m) Vec8<T>::load(x + b + (v0s[j] + m * map.px) * 8, nx[j][m]);
       }
   };
-  if (warp < units) fetch(warp);
-  for (size_t u = warp; u < units; u += nwarps) {
+  if (first < units) fetch(first);
+  for (size_t u0 = first; u0 < units; u0 += stride) {
+    const bool live = u0 + sub < units;
+    const size_t u = live ? u0 + sub : units - 1;
     const size_t row = u / heads;
     const int h = (int)(u - row * heads);
     const size_t base = row * d + (size_t)h * D;
@@ -570,7 +650,7 @@ __global__ void __launch_bounds__(256) fw_qk_prep_fwd_warp_kernel(
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int i = 0; i < 8; ++i) s[j][m][i] = nx[j][m][i];
-    if (u + nwarps < units) fetch(u + nwarps);
+    if (u0 + stride < units) fetch(u0 + stride);
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < MAXP; ++j) {
@@ -596,9 +676,10 @@ __global__ void __launch_bounds__(256) fw_qk_prep_fwd_warp_kernel(
     }
     float inv = 1.f;
     if (norm) {
-      ss = warp_sum(ss);
+      ss = group_sum<G>(ss);
       inv = norm == 1 ? 1.f / (sqrtf(ss) + 1e-5f) : rsqrtf(ss / D + 1e-5f);
     }
+    if (!live) continue;                       // no shuffles below
     if (lane == 0) inv_out[u] = inv;
     const int pos = offset + (int)(row % l);
 #pragma unroll
@@ -632,10 +713,10 @@ __global__ void __launch_bounds__(256) fw_qk_prep_fwd_warp_kernel(
   }
 }
 
-// A warp keeps one head (warp index modulo heads) and strides over the rows, so its lanes own fixed columns and
+// A lane group keeps one head (group index modulo heads) and strides over the rows, so its lanes own fixed columns and
 // carry the d(scale) / d(shift) partial sums in registers; they are merged per block in shared memory and added
 // to the result with one atomic per column and block.
-template <typename T, int MAXP>
+template <typename T, int MAXP, int G>
 __global__ void __launch_bounds__(256) fw_qk_prep_bwd_warp_kernel(
     const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ scale, const T* __restrict__ shift,
     const float* __restrict__ inv_in, const float2* __restrict__ table, T* __restrict__ dx,
@@ -644,15 +725,16 @@ __global__ void __launch_bounds__(256) fw_qk_prep_bwd_warp_kernel(
   extern __shared__ float red[];                 // [2][d] block sums of d(scale), d(shift)
   const int D = d / heads;
   const QkPairMap map(D, rope_dim);
-  const int lane = threadIdx.x & 31;
-  const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;      // a multiple of heads (host)
-  const int h = (int)(warp % heads);
+  const int lane = threadIdx.x & (G - 1);
+  const size_t group = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const size_t first_group = ((size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / G;     // of this warp
+  const size_t stride = (size_t)gridDim.x * blockDim.x / G / heads;      // the group count is a multiple of heads (host)
+  const int h = (int)(group % heads);
   const int half = rope_dim >> 1;
   int v0s[MAXP], toff[MAXP];                      // per lane: first vector of each owned pair, its table offset
 #pragma unroll
   for (int j = 0; j < MAXP; ++j) {
-    const int p = lane + 32 * j;
+    const int p = lane + G * j;
     v0s[j] = p < map.npairs ? map.first_vec(p) : -1;
     toff[j] = (p % map.px) * 8;
   }
@@ -681,7 +763,10 @@ __global__ void __launch_bounds__(256) fw_qk_prep_bwd_warp_kernel(
       }
     }
   };
-  for (size_t row = warp / heads; row < rows; row += nwarps / heads) {
+  size_t my_row = group / heads;
+  for (size_t row0 = first_group / heads; row0 < rows; row0 += stride, my_row += stride) {
+    const bool live = my_row < rows;
+    const size_t row = live ? my_row : rows - 1;
     const size_t base = row * d + (size_t)h * D;
     const int pos = offset + (int)(row % l);
     float dn[MAXP][2][8], xv[MAXP][2][8];
@@ -727,10 +812,11 @@ __global__ void __launch_bounds__(256) fw_qk_prep_bwd_warp_kernel(
     const float inv = inv_in[row * heads + h];
     float c1 = 0.f;                              // coefficient of s in d(s)
     if (norm) {
-      dot = warp_sum(dot);
+      dot = group_sum<G>(dot);
       if (norm == 1) c1 = dot * inv * inv / fmaxf(1.f / inv - 1e-5f, 1e-20f);
       else c1 = dot * inv * inv * inv / D;
     }
+    if (!live) continue;                         // no shuffles below
 #pragma unroll
     for (int j = 0; j < MAXP; ++j) {
       if (v0s[j] >= 0) {
@@ -801,16 +887,18 @@ std::vector<at::Tensor> fw_qk_prep_fwd(at::Tensor x, c10::optional<at::Tensor> s
   size_t smem = (d + heads) * sizeof(float);
   if (qk_warp_form_ok(d, (int)heads, (int)rope_dim) && rows > 0) {
     const size_t units = (size_t)rows * heads;
-    const int blocks = (int)std::max<size_t>(1, std::min<size_t>((units + 7) / 8, (size_t)sm_count() * 8));
+    const int pairs = d / (int)heads / 16;
     UTTT_DISPATCH_FLOAT(x, {
-      auto go = [&](auto kernel) {
+      auto go = [&](auto kernel, int lanes) {
+        const size_t per_block = 8 * (32 / lanes);
+        const int blocks = (int)std::max<size_t>(1, std::min<size_t>((units + per_block - 1) / per_block, (size_t)sm_count() * 8));
         kernel<<<blocks, 256, 0, cur_stream()>>>(
             ptr<T>(x), sc.defined() ? ptr<T>(sc) : nullptr, sc.defined() ? ptr<T>(sh) : nullptr,
             rope_dim > 0 ? reinterpret_cast<const float2*>(table.data_ptr()) : nullptr, ptr<T>(y), ptr<float>(inv),
             (size_t)rows, d, (int)heads, (int)rope_dim, (int)offset, (int)l, silu ? 1 : 0, (int)norm);
       };
-      if (d / heads <= 512) go(fw_qk_prep_fwd_warp_kernel<T, 1>);
-      else go(fw_qk_prep_fwd_warp_kernel<T, 2>);
+      if (pairs <= 32) with_lanes(pairs, [&](auto g) { go(fw_qk_prep_fwd_warp_kernel<T, 1, decltype(g)::value>, g); });
+      else go(fw_qk_prep_fwd_warp_kernel<T, 2, 32>, 32);
     });
     count_launch();
     return {y, inv};
@@ -844,20 +932,22 @@ std::vector<at::Tensor> fw_qk_prep_bwd(at::Tensor dy, at::Tensor x, c10::optiona
   size_t smem = (2 * d + heads) * sizeof(float);
   int blocks = std::max(1, std::min(rows, sm_count() * 4));
   if (qk_warp_form_ok(d, (int)heads, (int)rope_dim) && rows > 0 && heads <= 8 * 4) {
-    // 8 warps per block; the warp count must be a multiple of the head count (a warp keeps its head)
-    int wblocks = std::max(1, std::min((int)(((size_t)rows * heads + 7) / 8), sm_count() * 4));
-    while (((size_t)wblocks * 8) % heads != 0) ++wblocks;
+    const int pairs = d / (int)heads / 16;
     const size_t wsmem = (size_t)2 * d * sizeof(float);
     UTTT_DISPATCH_FLOAT(x, {
-      auto go = [&](auto kernel) {
+      auto go = [&](auto kernel, int lanes) {
+        // the number of lane groups must be a multiple of the head count (a group keeps its head)
+        const size_t per_block = 256 / lanes;
+        int wblocks = (int)std::max<size_t>(1, std::min<size_t>(((size_t)rows * heads + per_block - 1) / per_block, (size_t)sm_count() * 4));
+        while (((size_t)wblocks * per_block) % heads != 0) ++wblocks;
         kernel<<<wblocks, 256, has ? wsmem : 0, cur_stream()>>>(
             ptr<T>(dy), ptr<T>(x), has ? ptr<T>(sc) : nullptr, has ? ptr<T>(sh) : nullptr, ptr<float>(inv),
             rope_dim > 0 ? reinterpret_cast<const float2*>(table.data_ptr()) : nullptr, ptr<T>(dx),
             has ? ptr<float>(dscale) : nullptr, has ? ptr<float>(dshift) : nullptr, (size_t)rows, d, (int)heads,
             (int)rope_dim, (int)offset, (int)l, silu ? 1 : 0, (int)norm);
       };
-      if (d / heads <= 512) go(fw_qk_prep_bwd_warp_kernel<T, 1>);
-      else go(fw_qk_prep_bwd_warp_kernel<T, 2>);
+      if (pairs <= 32) with_lanes(pairs, [&](auto g) { go(fw_qk_prep_bwd_warp_kernel<T, 1, decltype(g)::value>, g); });
+      else go(fw_qk_prep_bwd_warp_kernel<T, 2, 32>, 32);
     });
     count_launch();
     return {dx, dscale, dshift};
@@ -1123,15 +1213,14 @@ __device__ __forceinline__ bool zero_pad_block(void* out, int vec_per_row, const
   return true;
 }
 
-template <typename T>
+template <typename T, int G>
 __global__ void permute_rows_kernel(const T* __restrict__ x, const int64_t* __restrict__ dest,
                                     const float* __restrict__ w, T* __restrict__ out, size_t n_copies, int k,
                                     int d, long long rows_out, int* __restrict__ status, PadLayout pad) {
   if (zero_pad_block(out, d * (int)sizeof(T) / 16, pad)) return;
-  size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  size_t nwarps = ((size_t)pad.copy_blocks * blockDim.x) >> 5;
-  for (size_t c = warp; c < n_copies; c += nwarps) {
+  const int lane = threadIdx.x & (G - 1);
+  const size_t ngroups = (size_t)pad.copy_blocks * blockDim.x / G;
+  for (size_t c = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G; c < n_copies; c += ngroups) {
     if (!UTTT_INDEX_OK(dest[c], rows_out, status, 71)) continue;
     const T* src = x + (c / k) * d;
     T* dst = out + (size_t)dest[c] * d;
@@ -1139,10 +1228,10 @@ __global__ void permute_rows_kernel(const T* __restrict__ x, const int64_t* __re
       constexpr int per = 16 / sizeof(T);   // elements per uint4
       const uint4* s4 = reinterpret_cast<const uint4*>(src);
       uint4* d4 = reinterpret_cast<uint4*>(dst);
-      for (int v = lane; v < d / per; v += 32) d4[v] = s4[v];
+      for (int v = lane; v < d / per; v += G) d4[v] = s4[v];
     } else {
       float wj = w[c];
-      for (int v = lane; v < (d >> 3); v += 32) {
+      for (int v = lane; v < (d >> 3); v += G) {
         float f[8];
         Vec8<T>::load(src + v * 8, f);
 #pragma unroll
@@ -1154,21 +1243,20 @@ __global__ void permute_rows_kernel(const T* __restrict__ x, const int64_t* __re
 }
 
 // out[i] = sum_j w[i,j] * y[dest[i,j]]
-template <typename T>
+template <typename T, int G>
 __global__ void unpermute_rows_kernel(const T* __restrict__ y, const int64_t* __restrict__ dest,
                                       const float* __restrict__ w, T* __restrict__ out, size_t rows, int k, int d,
                                       long long rows_in, int* __restrict__ status) {
-  size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
-  int nv = d >> 3;
-  for (size_t r = warp; r < rows; r += nwarps) {
+  const int lane = threadIdx.x & (G - 1);
+  const size_t ngroups = (size_t)gridDim.x * blockDim.x / G;
+  const int nv = d >> 3;
+  for (size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G; r < rows; r += ngroups) {
 #ifdef UTTT_BOUNDS_CHECK
     bool in_range = true;
     for (int j = 0; j < k; ++j) in_range = UTTT_INDEX_OK(dest[r * k + j], rows_in, status, 72) && in_range;
     if (!in_range) continue;
 #endif
-    for (int v = lane; v < nv; v += 32) {
+    for (int v = lane; v < nv; v += G) {
       float acc[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -1185,23 +1273,24 @@ __global__ void unpermute_rows_kernel(const T* __restrict__ y, const int64_t* __
 }
 
 // dy[dest[i,j]] = w[i,j] * dout[i];  dw[i,j] = <y[dest[i,j]], dout[i]>
-template <typename T>
+template <typename T, int G>
 __global__ void unpermute_rows_bwd_kernel(const T* __restrict__ dout, const T* __restrict__ y,
                                           const int64_t* __restrict__ dest, const float* __restrict__ w,
                                           T* __restrict__ dy, float* __restrict__ dw, size_t n_copies, int k, int d,
                                           PadLayout pad, long long rows_in, int* __restrict__ status) {
   if (zero_pad_block(dy, d * (int)sizeof(T) / 16, pad)) return;
-  size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  size_t nwarps = ((size_t)pad.copy_blocks * blockDim.x) >> 5;
-  int nv = d >> 3;
-  for (size_t c = warp; c < n_copies; c += nwarps) {
-    size_t r = c / k;
-    if (!UTTT_INDEX_OK(dest[c], rows_in, status, 72)) continue;
+  const int lane = threadIdx.x & (G - 1), sub = (threadIdx.x & 31) / G;
+  const size_t first = (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 / G);
+  const size_t stride = (size_t)pad.copy_blocks * blockDim.x / G;
+  const int nv = d >> 3;
+  for (size_t c0 = first; c0 < n_copies; c0 += stride) {
+    const size_t c = min(c0 + sub, n_copies - 1);
+    const size_t r = c / k;
+    const bool live = c0 + sub < n_copies && UTTT_INDEX_OK(dest[c], rows_in, status, 72);
     size_t dr = (size_t)dest[c];
     float wj = w[c];
     float dot = 0.f;
-    for (int v = lane; v < nv; v += 32) {
+    for (int v = lane; live && v < nv; v += G) {
       float g[8], f[8], o[8];
       Vec8<T>::load(dout + r * d + v * 8, g);
       Vec8<T>::load(y + dr * d + v * 8, f);
@@ -1212,8 +1301,8 @@ __global__ void unpermute_rows_bwd_kernel(const T* __restrict__ dout, const T* _
       }
       Vec8<T>::store(dy + dr * d + v * 8, o);
     }
-    dot = warp_sum(dot);
-    if (lane == 0) dw[c] = dot;
+    dot = group_sum<G>(dot);
+    if (lane == 0 && live) dw[c] = dot;
   }
 }
 
@@ -1233,6 +1322,13 @@ static at::Tensor padded_buffer(int64_t rows_padded, int d, const at::TensorOpti
   return out;
 }
 
+// rows of d elements that a block of 256 threads moves at a time
+static inline int copies_per_block(int d) {
+  int n = 0;
+  with_lanes(d / 8, [&](auto g) { n = 256 / decltype(g)::value; });
+  return n;
+}
+
 at::Tensor permute_rows(at::Tensor x, at::Tensor dest, int64_t rows_padded, c10::optional<at::Tensor> w,
                         c10::optional<at::Tensor> offsets, c10::optional<at::Tensor> sizes) {
   c10::cuda::CUDAGuard guard(x.device());
@@ -1240,15 +1336,18 @@ at::Tensor permute_rows(at::Tensor x, at::Tensor dest, int64_t rows_padded, c10:
   int k = dest.size(1);
   TORCH_CHECK(x.is_contiguous() && dest.is_contiguous() && dest.scalar_type() == at::kLong && d % 8 == 0);
   size_t n = (size_t)dest.numel();
-  int blocks = (int)std::max<size_t>(1, std::min<size_t>((n + 7) / 8, (size_t)sm_count() * 16));
+  const int per_block = copies_per_block(d);
+  int blocks = (int)std::max<size_t>(1, std::min<size_t>((n + per_block - 1) / per_block, (size_t)sm_count() * 16));
   PadLayout pad;
   auto out = padded_buffer(rows_padded, d, x.options(), offsets, sizes, blocks, &pad);
   at::Tensor wf;
   if (w.has_value() && w->defined()) wf = w->to(at::kFloat).contiguous();
   UTTT_DISPATCH_FLOAT(x, {
-    permute_rows_kernel<T><<<blocks + 2 * pad.groups, 256, 0, cur_stream()>>>(
-        ptr<T>(x), ptr<int64_t>(dest), wf.defined() ? ptr<float>(wf) : nullptr, ptr<T>(out), n, k, d,
-        (long long)rows_padded, gemm_status(x).data_ptr<int>(), pad);
+    with_lanes(d / 8, [&](auto g) {
+      permute_rows_kernel<T, decltype(g)::value><<<blocks + 2 * pad.groups, 256, 0, cur_stream()>>>(
+          ptr<T>(x), ptr<int64_t>(dest), wf.defined() ? ptr<float>(wf) : nullptr, ptr<T>(out), n, k, d,
+          (long long)rows_padded, gemm_status(x).data_ptr<int>(), pad);
+    });
   });
   count_launch();
   return out;
@@ -1263,12 +1362,14 @@ at::Tensor unpermute_rows(at::Tensor y, at::Tensor dest, c10::optional<at::Tenso
   at::Tensor wf;
   if (w.has_value() && w->defined()) wf = w->to(at::kFloat).contiguous();
   auto out = at::empty({(int64_t)rows, d}, y.options());
-  int blocks = (int)std::max<size_t>(1, std::min<size_t>((rows + 7) / 8, (size_t)sm_count() * 16));
+  const int per_block = copies_per_block(d);
+  int blocks = (int)std::max<size_t>(1, std::min<size_t>((rows + per_block - 1) / per_block, (size_t)sm_count() * 16));
   UTTT_DISPATCH_FLOAT(y, {
-    unpermute_rows_kernel<T><<<blocks, 256, 0, cur_stream()>>>(ptr<T>(y), ptr<int64_t>(dest),
-                                                              wf.defined() ? ptr<float>(wf) : nullptr, ptr<T>(out),
-                                                              rows, k, d, (long long)y.size(0),
-                                                              gemm_status(y).data_ptr<int>());
+    with_lanes(d / 8, [&](auto g) {
+      unpermute_rows_kernel<T, decltype(g)::value><<<blocks, 256, 0, cur_stream()>>>(
+          ptr<T>(y), ptr<int64_t>(dest), wf.defined() ? ptr<float>(wf) : nullptr, ptr<T>(out), rows, k, d,
+          (long long)y.size(0), gemm_status(y).data_ptr<int>());
+    });
   });
   count_launch();
   return out;
@@ -1281,14 +1382,17 @@ std::vector<at::Tensor> unpermute_rows_bwd(at::Tensor dout, at::Tensor y, at::Te
   int k = dest.size(1);
   size_t n = (size_t)dest.numel();
   auto wf = w.to(at::kFloat).contiguous();
-  int blocks = (int)std::max<size_t>(1, std::min<size_t>((n + 7) / 8, (size_t)sm_count() * 16));
+  const int per_block = copies_per_block(d);
+  int blocks = (int)std::max<size_t>(1, std::min<size_t>((n + per_block - 1) / per_block, (size_t)sm_count() * 16));
   PadLayout pad;
   auto dy = padded_buffer(y.size(0), d, y.options(), offsets, sizes, blocks, &pad);
   auto dw = at::empty({dest.size(0), k}, y.options().dtype(at::kFloat));
   UTTT_DISPATCH_FLOAT(y, {
-    unpermute_rows_bwd_kernel<T><<<blocks + 2 * pad.groups, 256, 0, cur_stream()>>>(
-        ptr<T>(dout), ptr<T>(y), ptr<int64_t>(dest), ptr<float>(wf), ptr<T>(dy), ptr<float>(dw), n, k, d, pad,
-        (long long)y.size(0), gemm_status(y).data_ptr<int>());
+    with_lanes(d / 8, [&](auto g) {
+      unpermute_rows_bwd_kernel<T, decltype(g)::value><<<blocks + 2 * pad.groups, 256, 0, cur_stream()>>>(
+          ptr<T>(dout), ptr<T>(y), ptr<int64_t>(dest), ptr<float>(wf), ptr<T>(dy), ptr<float>(dw), n, k, d, pad,
+          (long long)y.size(0), gemm_status(y).data_ptr<int>());
+    });
   });
   count_launch();
   return {dy, dw};
@@ -1315,35 +1419,53 @@ __global__ void plan_count_kernel(const int* __restrict__ idx, int* __restrict__
 // single CTA: per-group sizes, per-block exclusive offsets inside each group, padded group offsets, tile table
 __global__ void plan_scan_kernel(int* __restrict__ blk_counts, int* __restrict__ sizes, int* __restrict__ offsets,
                                  int* __restrict__ tile_group, int B, int E, int nblk, int t_max) {
-  int G = B * E;
+  // Latency-bound (one block, a few KB): the per-block counts of a group are fetched eight at a time, the group starts
+  // are a block-wide scan over 1024 groups at a time.
+  const int G = B * E;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ int warp_total[32];
   __shared__ int carry;
-  for (int g = threadIdx.x; g < G; g += blockDim.x) {
-    int b = g / E, e = g % E;
-    int run = 0;
-    for (int blk = 0; blk < nblk; ++blk) {
-      size_t at = ((size_t)b * nblk + blk) * E + e;
-      int c = blk_counts[at];
-      blk_counts[at] = run;            // exclusive offset of this block inside the group
-      run += c;
-    }
-    sizes[g] = run;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int g = 0; g < G; ++g) {
-      offsets[g] = acc;
-      acc += (sizes[g] + 127) / 128 * 128;
-    }
-    offsets[G] = acc;
-    carry = acc;
-  }
-  __syncthreads();
+  if (threadIdx.x == 0) carry = 0;
   for (int t = threadIdx.x; t < t_max; t += blockDim.x) tile_group[t] = -1;
   __syncthreads();
-  for (int g = threadIdx.x; g < G; g += blockDim.x) {
-    for (int t = offsets[g] / 128; t < offsets[g + 1] / 128; ++t) tile_group[t] = g;
+  for (int g0 = 0; g0 < G; g0 += blockDim.x) {
+    const int g = g0 + threadIdx.x;
+    int run = 0;
+    if (g < G) {
+      const size_t at = (size_t)(g / E) * nblk * E + g % E;
+      for (int blk0 = 0; blk0 < nblk; blk0 += 8) {
+        int c[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) c[i] = blk0 + i < nblk ? blk_counts[at + (size_t)(blk0 + i) * E] : 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (blk0 + i < nblk) blk_counts[at + (size_t)(blk0 + i) * E] = run;   // exclusive offset inside the group
+          run += c[i];
+        }
+      }
+      sizes[g] = run;
+    }
+    const int padded = (run + 127) / 128 * 128;
+    int incl = padded;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) warp_total[warp] = incl;
+    __syncthreads();
+    int before = carry;
+    for (int w = 0; w < warp; ++w) before += warp_total[w];
+    const int start = before + incl - padded;
+    if (g < G) {
+      offsets[g] = start;
+      for (int t = start / 128; t < (start + padded) / 128; ++t) tile_group[t] = g;
+    }
+    __syncthreads();                                  // everyone has read carry and the warp totals
+    if (threadIdx.x == blockDim.x - 1) carry = before + incl;
+    __syncthreads();
   }
+  if (threadIdx.x == 0) offsets[G] = carry;
 }
 
 __global__ void plan_dest_kernel(const int* __restrict__ idx, const int* __restrict__ blk_offsets,
