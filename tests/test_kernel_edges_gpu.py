@@ -160,3 +160,30 @@ def test_group_plan_scan(bsz, n, e, k):
     for a, b in ((plan.dest, dest), (plan.offsets, offsets), (plan.sizes, sizes), (plan.tile_group, tile_group)):
         assert torch.equal(a.cpu().long(), b.cpu().long())
     assert plan.rows_padded == rows
+
+
+# Expert counts of every accumulator width, one slab and several, the largest pair that fits and one that does not
+# (general kernel), fewer rows than a tile, sequences that end inside a tile.
+@pytest.mark.parametrize("e,d", [(16, 64), (16, 512), (32, 192), (48, 384), (48, 512), (64, 64), (64, 192), (64, 512), (24, 128)])
+@pytest.mark.parametrize("kind", ["softmax", "norm_softmax", "norm_relu"])
+@pytest.mark.parametrize("bsz,n,topk", [(1, 5, 1), (3, 1003, 4)])
+def test_router_matches_double_precision(e, d, kind, bsz, n, topk):
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(e + d + n)
+    rows = torch.randn(bsz, n, d, generator=gen, device=DEV).bfloat16()
+    router = torch.randn(e, d, generator=gen, device=DEV) * d ** -0.5
+    bias = torch.randn(e, generator=gen, device=DEV) * 0.02
+    idx, w, psum = ops.route_topk(rows, router, bias, topk, 0.7, False, False, kind, 0.0, 1e-6)
+    _status_ok()
+    sel, probs = ref.route_scores(rows.double() @ router.double().t(), kind, 0.0, 1e-6)
+    score = sel + bias.double()
+    top = torch.topk(score, topk + 1, dim=-1).values
+    gap = 1e-4                                                   # fp32 sums of d products of size one
+    clear = top[..., topk - 1] - top[..., topk] > gap
+    chosen = torch.zeros(bsz, n, e, device=DEV, dtype=torch.bool).scatter_(2, idx.long(), True)
+    assert bool((chosen.sum(-1) == topk).all())
+    assert bool(((score >= top[..., topk - 1:topk] - gap) | ~chosen).all())
+    assert bool((chosen == (score >= top[..., topk - 1:topk]))[clear].all())
+    # fp32 logits: d 2^-24 of their size at most; __expf adds 2^-21 of its argument
+    torch.testing.assert_close(w.view(bsz, n, topk).double(), probs.gather(-1, idx.long()) * 0.7, atol=2e-6, rtol=1e-4)
+    torch.testing.assert_close(psum.double(), probs.sum(1), atol=1e-4, rtol=1e-4)

@@ -10,7 +10,7 @@
 //   weight = alpha * probs[idx]   or   alpha * probs[idx] / sum_sel probs[idx]
 //   probs_sum[b, e] += probs[r, e]                            (load-balance statistics per sequence)
 //
-// Forward: a block stages 64 rows in shared memory, each warp multiplies 8 of them with lane = expert (two
+// Forward, bf16 rows: tensor cores (router_fwd_tc_kernel).  Other row types and shapes: a block stages 64 rows in shared memory, each warp multiplies 8 of them with lane = expert (two
 // experts per lane when E = 64) against the transposed router matrix in shared memory, then does the softmax
 // and the top-k with warp shuffles.
 // Backward: one kernel turns (d weight, d probs_sum) into d logits and d rows (lane = slice of D), a second one
@@ -23,8 +23,13 @@
 #include <torch/extension.h>
 
 #include "common.cuh"
+#include "ptx.cuh"
+#include "tc_gemm.cuh"
 
 namespace uttt {
+
+at::Tensor gemm_status(at::Tensor like);
+at::Tensor col_sum(at::Tensor partial);
 
 constexpr int kMaxTopK = 4;
 
@@ -234,6 +239,277 @@ __global__ void __launch_bounds__(256) router_fwd_kernel(const T* __restrict__ r
     }
   }
   flush();
+}
+
+// ------------------------------------------------------------------------------------ forward on tensor cores
+// logits[r, e] = <x[r], w[e]> with x in bf16 and w in fp32: w is the sum of three bf16 numbers (8 + 8 + 8 significant
+// bits; what is left is below 2^-26 |w|), products of bf16 numbers are exact in fp32, and the three products are added
+// into one fp32 accumulator.  So the tensor core gives the fp32 result at three bf16 products, and a thread owns a
+// whole row of logits: softmax and top-k need no shuffles.
+//   warp 8 / lane 0 : TMA producer, 64-column slabs of 128 rows -> ring
+//   warp 9 / lane 0 : MMA issuer, accumulators of two tiles in flight
+//   warps 0-3, 4-7  : softmax, top-k and balance sums of every other tile, thread = row
+// One persistent block per SM; the three parts of the router stay in shared memory, swizzled as the B operand.  The
+// general kernel is bound by its fp32 multiply-adds and their shared-memory reads.  196,608 rows of 64, 64 experts:
+// 57 -> 8 us; 16,384 rows of 384, 32 experts: 46 -> 10 us; 4 rows of 192, 16 experts: 16 -> 7 us.  The logits' error
+// against 64 bits is that of the general kernel (both below 1e-6 of their size).
+constexpr int kRtStages = 4;
+constexpr int kRtSlab = 128 * 128;               // 128 rows x 64 bf16
+constexpr int kRtPad = 4;                        // floats between staged probability rows: conflict-free 16-byte access
+
+struct RouterTcParams {
+  const float* router;
+  const float* bias;
+  int R, D, topk, rows_per_batch;
+  float alpha;
+  int bias_in_logits, renorm, mode;
+  float rscale, norm_eps;
+  int* idx;
+  float* w;
+  float* probs;
+  float* probs_sum;
+  float* logits;
+  int* status;
+};
+
+__host__ __device__ constexpr int router_tc_smem(int D, int E) {
+  return 3 * D * E * 2 + kRtStages * kRtSlab + 2 * 128 * (E + kRtPad) * 4 + 2 * E * 4 + 256 + 1024;
+}
+
+template <int E>
+__global__ void __launch_bounds__(320, 1) router_fwd_tc_kernel(const __grid_constant__ CUtensorMap tx, RouterTcParams p) {
+  extern __shared__ uint8_t smem_t[];
+  const uint32_t base = (ptx::smem_u32(smem_t) + 1023u) & ~1023u;
+  uint8_t* gen = smem_t + (base - ptx::smem_u32(smem_t));
+  const int slabs = p.D / 64;
+  const uint32_t part_bytes = (uint32_t)slabs * E * 128;            // one part of the router: [slab][E rows x 128 bytes]
+  const uint32_t ring = base + 3 * part_bytes;
+  const uint32_t stage_off = 3 * part_bytes + kRtStages * kRtSlab;
+  float* bias_s = reinterpret_cast<float*>(gen + stage_off + 2 * 128 * (E + kRtPad) * 4);      // [2][E]: logits, selection
+  const uint32_t bars = base + stage_off + 2 * 128 * (E + kRtPad) * 4 + 2 * E * 4;
+  auto full = [&](int s) { return bars + 8 * s; };
+  auto empty = [&](int s) { return bars + 32 + 8 * s; };
+  auto acc_full = [&](int g) { return bars + 64 + 8 * g; };
+  auto acc_empty = [&](int g) { return bars + 80 + 8 * g; };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + (bars - base) + 96);
+  const int warp = ptx::warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
+  const int tiles = (p.R + 127) / 128;
+  {
+    __shared__ int prior_failure;
+    if (threadIdx.x == 0) prior_failure = (p.status != nullptr) ? *(volatile int*)p.status : 0;
+    __syncthreads();
+    if (prior_failure != 0) return;
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kRtStages; ++s) {
+      ptx::mbar_init(full(s), 1);
+      ptx::mbar_init(empty(s), 1);
+    }
+    for (int g = 0; g < 2; ++g) {
+      ptx::mbar_init(acc_full(g), 1);
+      ptx::mbar_init(acc_empty(g), 128);
+    }
+    ptx::mbar_fence_init();
+    ptx::tma_prefetch_desc(&tx);
+  }
+  for (int i = threadIdx.x; i < E * (p.D / 8); i += blockDim.x) {
+    const int e = i / (p.D / 8), c8 = i % (p.D / 8);
+    float v[8];
+    Vec8<float>::load(p.router + (size_t)e * p.D + c8 * 8, v);
+    const uint32_t off = (uint32_t)(c8 >> 3) * (E * 128) + e * 128 + (((c8 & 7) ^ (e & 7)) << 4);
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+      Vec8<__nv_bfloat16>::store(reinterpret_cast<__nv_bfloat16*>(gen + part * part_bytes + off), v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] -= __bfloat162float(__float2bfloat16(v[k]));
+    }
+  }
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    const float b = p.bias != nullptr ? p.bias[e] : 0.f;
+    bias_s[e] = p.bias_in_logits ? b : 0.f;
+    bias_s[E + e] = p.bias_in_logits ? 0.f : b;
+  }
+  constexpr uint32_t kCols = E <= 16 ? 32 : E <= 32 ? 64 : 128;     // two accumulators of E columns, a power of two
+  constexpr uint32_t kAcc = kCols / 2;
+  if (warp == 8) {
+    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), kCols);
+    ptx::tmem_relinquish();
+  }
+  ptx::fence_proxy_async();                       // the router parts were written through the generic proxy
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem = ptx::warp_uniform(*tmem_slot);
+  constexpr uint32_t idesc = ptx::make_instr_desc(128, E, 0, 0);
+  bool ok = true;
+
+  if (warp == 8 && lane == 0) {
+    int it = 0;
+    for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      for (int kb = 0; kb < slabs; ++kb, ++it) {
+        const int s = it % kRtStages;
+        if (it >= kRtStages) ok = ptx::mbar_wait(empty(s), (it / kRtStages - 1) & 1, p.status, 81);
+        if (!ok) break;
+        ptx::mbar_expect_tx(full(s), kRtSlab);
+        ptx::tma_load_2d(ring + s * kRtSlab, &tx, full(s), kb * 64, t * 128);
+      }
+    }
+  } else if (warp == 9) {
+    int it = 0, n = 0;
+    for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++n) {
+      const int g = n & 1;
+      if (n >= 2) ok = ptx::warp_wait(acc_empty(g), ((n >> 1) - 1) & 1, p.status, 82);
+      if (!ok) break;
+      ptx::tc_fence_after_sync();
+      for (int kb = 0; kb < slabs; ++kb, ++it) {
+        const int s = it % kRtStages;
+        ok = ptx::warp_wait(full(s), (it / kRtStages) & 1, p.status, 83);
+        if (!ok) break;
+        ptx::tc_fence_after_sync();
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (int part = 2; part >= 0; --part) {   // small terms first
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const uint64_t da = ptx::make_smem_desc(ring + s * kRtSlab + k * 32, 16, 1024);
+              const uint64_t db = ptx::make_smem_desc(base + part * part_bytes + kb * (E * 128) + k * 32, 16, 1024);
+              ptx::mma_bf16_ss(tmem + g * kAcc, da, db, idesc, (kb > 0 || part < 2 || k > 0) ? 1u : 0u);
+            }
+          }
+          ptx::mma_commit(empty(s));
+        }
+      }
+      if (ok && ptx::elect_one()) ptx::mma_commit(acc_full(g));
+    }
+  } else if (warp < 8) {
+    const int g = warp >> 2, quarter = warp & 3, r_in = quarter * 32 + lane;
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    float* stage = reinterpret_cast<float*>(gen + stage_off) + g * 128 * (E + kRtPad);
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory"); };
+    // balance sums: thread = (expert column, strand of rows), carried over the tiles of a sequence
+    constexpr int kStrands = 128 / E, kStrandRows = 128 / kStrands;    // E = 48: 2 strands, 32 threads idle
+    const int col = r_in % E, strand = r_in / E;
+    float psum = 0.f;
+    int cur_b = -1;
+    int n = g;
+    for (int t = blockIdx.x + g * gridDim.x; t < tiles; t += 2 * gridDim.x, n += 2) {
+      // a failed wait must not leave part of the group at its barrier: the outcome is shared
+      bool got = ptx::mbar_wait(acc_full(g), (n >> 1) & 1, p.status, 84);
+      int all;
+      asm volatile(
+          "{\n\t.reg .pred P, Q;\n\tsetp.ne.b32 P, %1, 0;\n\tbarrier.cta.red.and.pred Q, %2, 128, P;\n\t"
+          "selp.b32 %0, 1, 0, Q;\n\t}"
+          : "=r"(all)
+          : "r"((int)got), "r"(1 + g)
+          : "memory");
+      if (!all) break;
+      ptx::tc_fence_after_sync();
+      const int row = t * 128 + r_in;
+      const bool live = row < p.R;
+      float lg[E];
+      {
+        uint32_t raw[E <= 16 ? 16 : E <= 32 ? 32 : 64];
+        if constexpr (E <= 16) ptx::tmem_ld_32x16(tmem + g * kAcc + lane_base, raw);
+        else if constexpr (E <= 32) ptx::tmem_ld_32x32(tmem + g * kAcc + lane_base, raw);
+        else ptx::tmem_ld_32x64(tmem + g * kAcc + lane_base, raw);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < E; ++e) lg[e] = __uint_as_float(raw[e]) + bias_s[e];
+      }
+      ptx::tc_fence_before_sync();
+      ptx::mbar_arrive(acc_empty(g));
+      if (p.mode != 0) {
+        // normalised variants: keep the raw logits for the backward, continue with the rescaled scores
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) ss = fmaf(lg[e], lg[e], ss);
+        const float inv_n = 1.f / fmaxf(sqrtf(ss), p.norm_eps);
+        if (live) {
+#pragma unroll
+          for (int e = 0; e < E; e += 4)
+            *reinterpret_cast<float4*>(p.logits + (size_t)row * E + e) = make_float4(lg[e], lg[e + 1], lg[e + 2], lg[e + 3]);
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const float z = lg[e] * inv_n;
+          lg[e] = (p.mode == 1 ? z : fmaxf(z, 0.f)) * p.rscale;
+        }
+      }
+      float mx = lg[0];
+#pragma unroll
+      for (int e = 1; e < E; ++e) mx = fmaxf(mx, lg[e]);
+      float pr[E], sum = 0.f;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        pr[e] = p.mode == 2 ? lg[e] : __expf(lg[e] - mx);
+        sum += pr[e];
+      }
+      float inv = 1.f / sum, uniform = 0.f;
+      if (p.mode == 2) {
+        if (sum > 0.f) inv = 1.f / fmaxf(sum, 1e-9f);
+        else { inv = 0.f; uniform = 1.f / (float)E; }
+      }
+#pragma unroll
+      for (int e = 0; e < E; ++e) pr[e] = fmaf(pr[e], inv, uniform);
+      // top-k by (logit + selection bias); ties go to the lower expert index
+      int pick_e[kMaxTopK];
+      float pick_p[kMaxTopK], psel = 0.f;
+      uint64_t taken = 0;
+#pragma unroll
+      for (int j = 0; j < kMaxTopK; ++j) {
+        if (j >= p.topk) break;
+        float bv = -INFINITY, bp = pr[0];
+        int be = 0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const float v = lg[e] + bias_s[E + e];
+          if (v > bv && !((taken >> e) & 1)) { bv = v; be = e; bp = pr[e]; }
+        }
+        taken |= 1ull << be;
+        pick_e[j] = be;
+        pick_p[j] = bp;
+        psel += bp;
+      }
+      if (live) {
+        const float scale = p.renorm ? p.alpha / fmaxf(psel, 1e-9f) : p.alpha;
+#pragma unroll
+        for (int j = 0; j < kMaxTopK; ++j) {
+          if (j >= p.topk) break;
+          p.idx[(size_t)row * p.topk + j] = pick_e[j];
+          p.w[(size_t)row * p.topk + j] = pick_p[j] * scale;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < E; e += 4)
+        *reinterpret_cast<float4*>(stage + r_in * (E + kRtPad) + e) = make_float4(pr[e], pr[e + 1], pr[e + 2], pr[e + 3]);
+      group_sync();
+      const int rows_here = min(128, p.R - t * 128);
+      for (int i = r_in; i < rows_here * (E / 4); i += 128) {
+        const int r = i / (E / 4), c = i % (E / 4);
+        reinterpret_cast<float4*>(p.probs)[(size_t)t * 128 * (E / 4) + i] =
+            *reinterpret_cast<const float4*>(stage + r * (E + kRtPad) + c * 4);
+      }
+      if (strand < kStrands) {
+        int r = strand * kStrandRows;
+        const int end = min(rows_here, r + kStrandRows);
+        while (r < end) {
+          const int b = (t * 128 + r) / p.rows_per_batch;
+          if (b != cur_b) {
+            if (cur_b >= 0) atomicAdd(p.probs_sum + (size_t)cur_b * E + col, psum);
+            psum = 0.f;
+            cur_b = b;
+          }
+          const int stop = (int)min((long long)end, (long long)(b + 1) * p.rows_per_batch - (long long)t * 128);
+          for (; r < stop; ++r) psum += stage[r * (E + kRtPad) + col];
+        }
+      }
+      group_sync();                               // the stage is free for the next tile
+    }
+    if (cur_b >= 0) atomicAdd(p.probs_sum + (size_t)cur_b * E + col, psum);
+  }
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 8) ptx::tmem_dealloc(tmem, kCols);
 }
 
 // ------------------------------------------------------------------------------------ backward: d logits, d rows
@@ -473,13 +749,35 @@ std::vector<at::Tensor> router_fwd(at::Tensor rows, at::Tensor router, c10::opti
   auto psum = at::zeros({R / rows_per_batch, E}, opts.dtype(at::kFloat));
   TORCH_CHECK(mode >= 0 && mode <= 2, "router mode: 0 softmax, 1 norm_softmax, 2 norm_relu");
   auto logits = mode != 0 ? at::empty({R, E}, opts.dtype(at::kFloat)) : at::empty({0}, opts.dtype(at::kFloat));
+  auto stream = at::cuda::getCurrentCUDAStream().stream();
+  // Tensor cores need whole 64-column slabs, an expert count that is an MMA width, and room for the three router parts.
+  const int tc_smem = router_tc_smem(D, E);
+  if (rows.scalar_type() == at::kBFloat16 && D % 64 == 0 && E % 16 == 0 && tc_smem <= 227 * 1024 - 64 && R > 0 &&
+      ((uintptr_t)rows.data_ptr() & 15) == 0 && ((uintptr_t)router.data_ptr() & 15) == 0) {
+    RouterTcParams tp{router.data_ptr<float>(), bp, R, D, (int)topk, (int)rows_per_batch, (float)alpha,
+                      bias_in_logits ? 1 : 0, renorm ? 1 : 0, (int)mode, (float)rscale, (float)norm_eps,
+                      idx.data_ptr<int>(), w.data_ptr<float>(), probs.data_ptr<float>(), psum.data_ptr<float>(),
+                      logits.data_ptr<float>(), gemm_status(rows).data_ptr<int>()};
+    auto tx = make_tmap_2d_bf16(rows.data_ptr(), R, D, 128, 64);
+    const int blocks = std::min((R + 127) / 128, sm_count());
+    auto launch = [&](auto kernel) {
+      C10_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem));
+      kernel<<<blocks, 320, tc_smem, stream>>>(tx, tp);
+      C10_CUDA_KERNEL_LAUNCH_CHECK();
+    };
+    if (E == 16) launch(router_fwd_tc_kernel<16>);
+    else if (E == 32) launch(router_fwd_tc_kernel<32>);
+    else if (E == 48) launch(router_fwd_tc_kernel<48>);
+    else launch(router_fwd_tc_kernel<64>);
+    count_launch();
+    return {idx, w, probs, psum, logits};
+  }
   const int epl = E > 32 ? 2 : 1;
   const bool bf = rows.scalar_type() == at::kBFloat16;
   const int rpw = bf ? 8 : 4;
   const size_t smem = (((size_t)D * (32 * epl + 1) * 4 + 15) & ~(size_t)15) + (size_t)8 * rpw * D * (bf ? 2 : 4);
   const int steps = (R + 8 * rpw - 1) / (8 * rpw);
   const int blocks = std::max(1, std::min(steps, 2 * sm_count()));
-  auto stream = at::cuda::getCurrentCUDAStream().stream();
   auto launch = [&](auto kernel, auto* rp) {
     C10_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<blocks, 256, smem, stream>>>(rp, router.data_ptr<float>(), bp, R, D, E, (int)topk, (int)rows_per_batch,
@@ -564,7 +862,9 @@ std::vector<at::Tensor> router_bwd(at::Tensor rows, at::Tensor router, at::Tenso
   }
   auto dlogits = at::empty({R, E}, probs.options());
   auto drows = need_drows ? at::empty_like(rows) : at::Tensor();
-  const int wchunk = 128;
+  // rows per block of the weight reduction: two blocks per SM when there are rows for them (each block writes an [E, D]
+  // partial sum, which at one block per 128 rows was as much traffic as the rows themselves)
+  const int wchunk = std::max(128, (R + 2 * sm_count() * 32 - 1) / (2 * sm_count() * 32) * 32);
   auto partial = at::empty({(R + wchunk - 1) / wchunk, E, D}, router.options());
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   const int dpl = (D + 31) / 32;
@@ -603,7 +903,7 @@ std::vector<at::Tensor> router_bwd(at::Tensor rows, at::Tensor router, at::Tenso
 #undef UTTT_ROUTER_BWD_W
   count_launch();
   count_launch();
-  auto drouter = partial.sum(0);
+  auto drouter = col_sum(partial);
   if (!need_drows) drows = at::empty({0}, rows.options());
   return {drows, drouter};
 }
