@@ -117,7 +117,7 @@ __global__ void __launch_bounds__((EPI != kEpiNone ? kFusedWarps : 4) * 32 + 64)
   auto acc_full = [&](int b) { return bar_base + 8u * (2 * STAGES + b); };
   auto acc_empty = [&](int b) { return bar_base + 8u * (2 * STAGES + 2 + b); };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_gen + L::kBarOffset + (2 * STAGES + 4) * 8);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
 
   {
     __shared__ int prior_failure;
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__((EPI != kEpiNone ? kFusedWarps : 4) * 32 + 64)
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = ptx::warp_uniform(*tmem_slot);
   OutT* out = reinterpret_cast<OutT*>(p.out);
   const int ldo = p.N;
 
@@ -226,28 +226,29 @@ __global__ void __launch_bounds__((EPI != kEpiNone ? kFusedWarps : 4) * 32 + 64)
       }
     }
   } else if (warp == EW + 1) {
-    if (lane == 0) {
-      // ================= MMA issuer =================
-      constexpr int a_mn = (MODE == kTN || MODE == kBTN) ? 1 : 0;
-      constexpr int b_mn = (MODE == kNN || MODE == kTN || MODE == kBNN || MODE == kBTN) ? 1 : 0;
-      constexpr uint32_t idesc = ptx::make_instr_desc(BM, BN, a_mn, b_mn);
-      uint32_t it = 0, acc_it = 0;
-      bool ok = true;
-      for (int id = blockIdx.x; id < total_tiles && ok; id += gridDim.x) {
-        TileCoord c = decode_tile<MODE, TW>(p, segs, id, tiles_n, tiles_m);
-        if (c.unused || c.nkb == 0) continue;
-        const int ab = acc_it & 1;
-        ok = ptx::mbar_wait(acc_empty(ab), ((acc_it >> 1) & 1) ^ 1, p.status, 22);
+    // ================= MMA issuer =================
+    constexpr int a_mn = (MODE == kTN || MODE == kBTN) ? 1 : 0;
+    constexpr int b_mn = (MODE == kNN || MODE == kTN || MODE == kBNN || MODE == kBTN) ? 1 : 0;
+    constexpr uint32_t idesc = ptx::make_instr_desc(BM, BN, a_mn, b_mn);
+    uint32_t it = 0, acc_it = 0;
+    bool ok = true;
+    for (int id = blockIdx.x; id < total_tiles && ok; id += gridDim.x) {
+      TileCoord c = decode_tile<MODE, TW>(p, segs, id, tiles_n, tiles_m);
+      const int nkb = ptx::warp_uniform(c.unused ? 0 : c.nkb);
+      if (nkb == 0) continue;
+      const int ab = acc_it & 1;
+      ok = ptx::warp_wait(acc_empty(ab), ((acc_it >> 1) & 1) ^ 1, p.status, 22);
+      if (!ok) break;
+      ptx::tc_fence_after_sync();
+      const uint32_t tmem_acc = tmem_base + ab * L::kAccStride;
+      for (int kb = 0; kb < nkb; ++kb, ++it) {
+        int s = it % STAGES;
+        ok = ptx::warp_wait(full_bar(s), (it / STAGES) & 1, p.status, 23);
         if (!ok) break;
         ptx::tc_fence_after_sync();
-        const uint32_t tmem_acc = tmem_base + ab * L::kAccStride;
-        for (int kb = 0; kb < c.nkb; ++kb, ++it) {
-          int s = it % STAGES;
-          ok = ptx::mbar_wait(full_bar(s), (it / STAGES) & 1, p.status, 23);
-          if (!ok) break;
-          ptx::tc_fence_after_sync();
-          uint32_t sa = smem_base + s * L::kStageBytes;
-          uint32_t sb = sa + L::kABytes;
+        uint32_t sa = smem_base + s * L::kStageBytes;
+        uint32_t sb = sa + L::kABytes;
+        if (ptx::elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             uint64_t da = a_mn ? ptx::make_smem_desc(sa + k * 2048, BK * 128, 1024)
@@ -258,10 +259,10 @@ __global__ void __launch_bounds__((EPI != kEpiNone ? kFusedWarps : 4) * 32 + 64)
           }
           ptx::mma_commit(empty_bar(s));
         }
-        if (!ok) break;
-        ptx::mma_commit(acc_full(ab));
-        ++acc_it;
       }
+      if (!ok) break;
+      if (ptx::elect_one()) ptx::mma_commit(acc_full(ab));
+      ++acc_it;
     }
   } else {
     // ================= epilogue (warps 0-3) =================
