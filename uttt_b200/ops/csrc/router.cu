@@ -814,7 +814,9 @@ static void launch_bwd_rows(int dpl, const float* router, const float* probs, co
                                           drows, mode, rscale, norm_eps, logits);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
   };
-  if (dpl <= 4) go(router_bwd_rows_kernel<T, EPL, 4, 8>, 8);
+  // slices of 32 columns per lane: with four of them for a head of 64 half of the multiply-adds were by zero
+  if (dpl <= 2) go(router_bwd_rows_kernel<T, EPL, 2, 8>, 8);
+  else if (dpl <= 4) go(router_bwd_rows_kernel<T, EPL, 4, 8>, 8);
   else if (dpl <= 8) go(router_bwd_rows_kernel<T, EPL, 8, 8>, 8);
   else if (dpl <= 12) go(router_bwd_rows_kernel<T, EPL, 12, 8>, 8);
   else go(router_bwd_rows_kernel<T, EPL, 16, 4>, 4);
@@ -830,7 +832,8 @@ static void launch_bwd_weight(int dpl, const T* rows, const float* dlogits, int 
     kernel<<<blocks, 256, smem, stream>>>(rows, dlogits, R, D, E, chunk, partial);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
   };
-  if (dpl <= 4) go(router_bwd_weight_kernel<T, EG, 4>);
+  if (dpl <= 2) go(router_bwd_weight_kernel<T, EG, 2>);
+  else if (dpl <= 4) go(router_bwd_weight_kernel<T, EG, 4>);
   else if (dpl <= 8) go(router_bwd_weight_kernel<T, EG, 8>);
   else if (dpl <= 12) go(router_bwd_weight_kernel<T, EG, 12>);
   else go(router_bwd_weight_kernel<T, EG, 16>);
