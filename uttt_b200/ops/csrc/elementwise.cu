@@ -39,8 +39,8 @@ static inline int sm_count() { return at::cuda::getCurrentDeviceProperties()->mu
 // there are more), so that a warp works on 32 / G narrow rows at once: a head of 64 elements has 8 vectors, and one
 // such row per warp leaves three lanes of four idle and a quarter of the bytes in flight.  The row loops are
 // warp-uniform (a group past the end repeats the last row and stores nothing), so the shuffles see full warps.
-// Heads of 64, 24,576 x 8 rows: memory preprocessing 20 -> 9 us forward, 48 -> 13 us backward.  Heads of 192, 2048 x 4
-// rows: 22 -> 20 us backward.
+// 196,608 rows of 64: memory preprocessing 99 -> 16 us, its backward 248 -> 34, norm 32 -> 11, its backward 82 -> 22,
+// scatter 22 -> 8, gather 26 -> 10.  8192 rows of 192: preprocessing 7.2 -> 4.8 us, its backward 13.7 -> 9.3.
 template <int G>
 __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
@@ -63,8 +63,8 @@ static inline void with_lanes(int vectors, F&& f) {
 }
 
 // out[c] = sum over p of partial[p, c]: the per-block partial sums of a kernel.  32 columns per block, 32 row strands
-// each, so that a few hundred partial rows are a handful of loads in flight per thread: 3.7 us for 592 x 768, where the
-// general reduction took 11.
+// each, so that a few hundred partial rows are a handful of loads in flight per thread: 4.2 us for 592 x 768, where the
+// general reduction took 15.7.
 __global__ void __launch_bounds__(1024) col_sum_kernel(const float* __restrict__ partial, float* __restrict__ out, int rows,
                                                        long long cols) {
   __shared__ float part[32][33];
@@ -1420,7 +1420,7 @@ __global__ void plan_count_kernel(const int* __restrict__ idx, int* __restrict__
 __global__ void plan_scan_kernel(int* __restrict__ blk_counts, int* __restrict__ sizes, int* __restrict__ offsets,
                                  int* __restrict__ tile_group, int B, int E, int nblk, int t_max) {
   // Latency-bound (one block, a few KB): the per-block counts of a group are fetched eight at a time, the group starts
-  // are a block-wide scan over 1024 groups at a time.
+  // are a block-wide scan over 1024 groups at a time (256 groups: 16 -> 5 us).
   const int G = B * E;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ int warp_total[32];
