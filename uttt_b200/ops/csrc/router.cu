@@ -251,8 +251,7 @@ __global__ void __launch_bounds__(256) router_fwd_kernel(const T* __restrict__ r
 //   warps 0-3, 4-7  : softmax, top-k and balance sums of every other tile, thread = row
 // One persistent block per SM; the three parts of the router stay in shared memory, swizzled as the B operand.  The
 // general kernel is bound by its fp32 multiply-adds and their shared-memory reads.  196,608 rows of 64, 64 experts:
-// 57 -> 8 us; 16,384 rows of 384, 32 experts: 46 -> 10 us; 4 rows of 192, 16 experts: 16 -> 7 us.  The logits' error
-// against 64 bits is that of the general kernel (both below 1e-6 of their size).
+// 234 -> 26 us.
 constexpr int kRtStages = 4;
 constexpr int kRtSlab = 128 * 128;               // 128 rows x 64 bf16
 constexpr int kRtPad = 4;                        // floats between staged probability rows: conflict-free 16-byte access
@@ -750,9 +749,11 @@ std::vector<at::Tensor> router_fwd(at::Tensor rows, at::Tensor router, c10::opti
   TORCH_CHECK(mode >= 0 && mode <= 2, "router mode: 0 softmax, 1 norm_softmax, 2 norm_relu");
   auto logits = mode != 0 ? at::empty({R, E}, opts.dtype(at::kFloat)) : at::empty({0}, opts.dtype(at::kFloat));
   auto stream = at::cuda::getCurrentCUDAStream().stream();
-  // Tensor cores need whole 64-column slabs, an expert count that is an MMA width, and room for the three router parts.
+  // Tensor cores for one 64-column slab and an expert count that is an MMA width.  The tensor core does not round its sums
+  // to nearest: the logits' relative error against 64 bits is 0.8e-7 at 64 columns (general kernel: 1.4e-7), but 5.3e-7
+  // at 192 (2.5e-7) and 1.1e-6 at 384 (3.5e-7), so wider rows keep the general kernel.
   const int tc_smem = router_tc_smem(D, E);
-  if (rows.scalar_type() == at::kBFloat16 && D % 64 == 0 && E % 16 == 0 && tc_smem <= 227 * 1024 - 64 && R > 0 &&
+  if (rows.scalar_type() == at::kBFloat16 && D == 64 && E % 16 == 0 && tc_smem <= 227 * 1024 - 64 && R > 0 &&
       ((uintptr_t)rows.data_ptr() & 15) == 0 && ((uintptr_t)router.data_ptr() & 15) == 0) {
     RouterTcParams tp{router.data_ptr<float>(), bp, R, D, (int)topk, (int)rows_per_batch, (float)alpha,
                       bias_in_logits ? 1 : 0, renorm ? 1 : 0, (int)mode, (float)rscale, (float)norm_eps,
@@ -814,7 +815,8 @@ static void launch_bwd_rows(int dpl, const float* router, const float* probs, co
                                           drows, mode, rscale, norm_eps, logits);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
   };
-  // slices of 32 columns per lane: with four of them for a head of 64 half of the multiply-adds were by zero
+  // slices of 32 columns per lane: with four of them for a head of 64 half of the multiply-adds were by zero (196,608
+  // rows, 64 experts: 194 -> 161 us)
   if (dpl <= 2) go(router_bwd_rows_kernel<T, EPL, 2, 8>, 8);
   else if (dpl <= 4) go(router_bwd_rows_kernel<T, EPL, 4, 8>, 8);
   else if (dpl <= 8) go(router_bwd_rows_kernel<T, EPL, 8, 8>, 8);
@@ -832,8 +834,7 @@ static void launch_bwd_weight(int dpl, const T* rows, const float* dlogits, int 
     kernel<<<blocks, 256, smem, stream>>>(rows, dlogits, R, D, E, chunk, partial);
     C10_CUDA_KERNEL_LAUNCH_CHECK();
   };
-  if (dpl <= 2) go(router_bwd_weight_kernel<T, EG, 2>);
-  else if (dpl <= 4) go(router_bwd_weight_kernel<T, EG, 4>);
+  if (dpl <= 4) go(router_bwd_weight_kernel<T, EG, 4>);
   else if (dpl <= 8) go(router_bwd_weight_kernel<T, EG, 8>);
   else if (dpl <= 12) go(router_bwd_weight_kernel<T, EG, 12>);
   else go(router_bwd_weight_kernel<T, EG, 16>);
