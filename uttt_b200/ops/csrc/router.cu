@@ -243,15 +243,18 @@ __global__ void __launch_bounds__(256) router_fwd_kernel(const T* __restrict__ r
 
 // ------------------------------------------------------------------------------------ forward on tensor cores
 // logits[r, e] = <x[r], w[e]> with x in bf16 and w in fp32: w is the sum of three bf16 numbers (8 + 8 + 8 significant
-// bits; what is left is below 2^-26 |w|), products of bf16 numbers are exact in fp32, and the three products are added
-// into one fp32 accumulator.  So the tensor core gives the fp32 result at three bf16 products, and a thread owns a
-// whole row of logits: softmax and top-k need no shuffles.
+// bits; what is left is below 2^-26 |w|), and products of bf16 numbers are exact in fp32.  The tensor core adds into its
+// fp32 accumulator without rounding to nearest, an error that grows with every addition, so each 64-column slab has an
+// accumulator of its own and the slabs are added in registers.  A thread owns a whole row of logits: softmax and top-k
+// need no shuffles.
 //   warp 8 / lane 0 : TMA producer, 64-column slabs of 128 rows -> ring
 //   warp 9 / lane 0 : MMA issuer, accumulators of two tiles in flight
 //   warps 0-3, 4-7  : softmax, top-k and balance sums of every other tile, thread = row
 // One persistent block per SM; the three parts of the router stay in shared memory, swizzled as the B operand.  The
-// general kernel is bound by its fp32 multiply-adds and their shared-memory reads.  196,608 rows of 64, 64 experts:
-// 234 -> 26 us.
+// general kernel is bound by its fp32 multiply-adds and their shared-memory reads.
+// 196,608 rows of 64, 64 experts: 234 -> 28 us; 16,384 of 384, 32 experts: 45 -> 10.5 us; 4 of 192, 16 experts: 15 -> 6 us.
+// Relative error of the logits against 64 bits (general kernel): 0.8e-7 (1.4e-7), 0.9e-7 (3.5e-7), 1.0e-7 (2.7e-7); with
+// one accumulator for all slabs it was 1.1e-6 at 384 columns.
 constexpr int kRtStages = 4;
 constexpr int kRtSlab = 128 * 128;               // 128 rows x 64 bf16
 constexpr int kRtPad = 4;                        // floats between staged probability rows: conflict-free 16-byte access
@@ -328,8 +331,8 @@ __global__ void __launch_bounds__(320, 1) router_fwd_tc_kernel(const __grid_cons
     bias_s[e] = p.bias_in_logits ? b : 0.f;
     bias_s[E + e] = p.bias_in_logits ? 0.f : b;
   }
-  constexpr uint32_t kCols = E <= 16 ? 32 : E <= 32 ? 64 : 128;     // two accumulators of E columns, a power of two
-  constexpr uint32_t kAcc = kCols / 2;
+  // two tiles in flight, a slab of a tile every kSlabCols columns (a load reads whole powers of two)
+  constexpr uint32_t kCols = 512, kAcc = kCols / 2, kSlabCols = E <= 16 ? 16 : E <= 32 ? 32 : 64;
   if (warp == 8) {
     ptx::tmem_alloc(ptx::smem_u32(tmem_slot), kCols);
     ptx::tmem_relinquish();
@@ -372,7 +375,7 @@ __global__ void __launch_bounds__(320, 1) router_fwd_tc_kernel(const __grid_cons
             for (int k = 0; k < 4; ++k) {
               const uint64_t da = ptx::make_smem_desc(ring + s * kRtSlab + k * 32, 16, 1024);
               const uint64_t db = ptx::make_smem_desc(base + part * part_bytes + kb * (E * 128) + k * 32, 16, 1024);
-              ptx::mma_bf16_ss(tmem + g * kAcc, da, db, idesc, (kb > 0 || part < 2 || k > 0) ? 1u : 0u);
+              ptx::mma_bf16_ss(tmem + g * kAcc + kb * kSlabCols, da, db, idesc, (part < 2 || k > 0) ? 1u : 0u);
             }
           }
           ptx::mma_commit(empty(s));
@@ -406,14 +409,16 @@ __global__ void __launch_bounds__(320, 1) router_fwd_tc_kernel(const __grid_cons
       const int row = t * 128 + r_in;
       const bool live = row < p.R;
       float lg[E];
-      {
-        uint32_t raw[E <= 16 ? 16 : E <= 32 ? 32 : 64];
-        if constexpr (E <= 16) ptx::tmem_ld_32x16(tmem + g * kAcc + lane_base, raw);
-        else if constexpr (E <= 32) ptx::tmem_ld_32x32(tmem + g * kAcc + lane_base, raw);
-        else ptx::tmem_ld_32x64(tmem + g * kAcc + lane_base, raw);
+#pragma unroll
+      for (int e = 0; e < E; ++e) lg[e] = bias_s[e];
+      for (int kb = 0; kb < slabs; ++kb) {
+        uint32_t raw[kSlabCols];
+        if constexpr (E <= 16) ptx::tmem_ld_32x16(tmem + g * kAcc + kb * kSlabCols + lane_base, raw);
+        else if constexpr (E <= 32) ptx::tmem_ld_32x32(tmem + g * kAcc + kb * kSlabCols + lane_base, raw);
+        else ptx::tmem_ld_32x64(tmem + g * kAcc + kb * kSlabCols + lane_base, raw);
         ptx::tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < E; ++e) lg[e] = __uint_as_float(raw[e]) + bias_s[e];
+        for (int e = 0; e < E; ++e) lg[e] += __uint_as_float(raw[e]);
       }
       ptx::tc_fence_before_sync();
       ptx::mbar_arrive(acc_empty(g));
@@ -749,11 +754,11 @@ std::vector<at::Tensor> router_fwd(at::Tensor rows, at::Tensor router, c10::opti
   TORCH_CHECK(mode >= 0 && mode <= 2, "router mode: 0 softmax, 1 norm_softmax, 2 norm_relu");
   auto logits = mode != 0 ? at::empty({R, E}, opts.dtype(at::kFloat)) : at::empty({0}, opts.dtype(at::kFloat));
   auto stream = at::cuda::getCurrentCUDAStream().stream();
-  // Tensor cores for one 64-column slab and an expert count that is an MMA width.  The tensor core does not round its sums
-  // to nearest: the logits' relative error against 64 bits is 0.8e-7 at 64 columns (general kernel: 1.4e-7), but 5.3e-7
-  // at 192 (2.5e-7) and 1.1e-6 at 384 (3.5e-7), so wider rows keep the general kernel.
+  // Tensor cores need whole 64-column slabs, an expert count that is an MMA width, room for the three router parts, and an
+  // accumulator per slab and tile.
   const int tc_smem = router_tc_smem(D, E);
-  if (rows.scalar_type() == at::kBFloat16 && D == 64 && E % 16 == 0 && tc_smem <= 227 * 1024 - 64 && R > 0 &&
+  const int slab_cols = E <= 16 ? 16 : E <= 32 ? 32 : 64;
+  if (rows.scalar_type() == at::kBFloat16 && D % 64 == 0 && E % 16 == 0 && tc_smem <= 227 * 1024 - 64 && D / 64 * slab_cols <= 256 && R > 0 &&
       ((uintptr_t)rows.data_ptr() & 15) == 0 && ((uintptr_t)router.data_ptr() & 15) == 0) {
     RouterTcParams tp{router.data_ptr<float>(), bp, R, D, (int)topk, (int)rows_per_batch, (float)alpha,
                       bias_in_logits ? 1 : 0, renorm ? 1 : 0, (int)mode, (float)rscale, (float)norm_eps,
@@ -866,9 +871,8 @@ std::vector<at::Tensor> router_bwd(at::Tensor rows, at::Tensor router, at::Tenso
   }
   auto dlogits = at::empty({R, E}, probs.options());
   auto drows = need_drows ? at::empty_like(rows) : at::Tensor();
-  // rows per block of the weight reduction: two blocks per SM when there are rows for them (each block writes an [E, D]
-  // partial sum, which at one block per 128 rows was as much traffic as the rows themselves)
-  const int wchunk = std::max(128, (R + 2 * sm_count() * 32 - 1) / (2 * sm_count() * 32) * 32);
+  // rows per block of the weight reduction; two long blocks per SM took 177 us at 196,608 rows of 64 where these take 137
+  const int wchunk = 128;
   auto partial = at::empty({(R + wchunk - 1) / wchunk, E, D}, router.options());
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   const int dpl = (D + 31) / 32;
