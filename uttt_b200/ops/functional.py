@@ -1512,6 +1512,19 @@ class _MomentumNormalize(torch.autograd.Function):
         if dz_new is None and dx is None:
             return None, None, None, None, None
         _, need_z, need_m = ctx.needs_input_grad[:3]
+        if torch.is_grad_enabled():
+            # somebody differentiates the gradient: the same formulas in operations that autograd sees
+            g = torch.zeros_like(z_new) if dz_new is None else dz_new
+            if dx is not None:
+                v, dxv = z_new.reshape(sumsq.numel(), -1), dx.to(z_new.dtype).reshape(sumsq.numel(), -1)
+                r = v.norm(dim=1, keepdim=True)
+                dot = (v * dxv).sum(1, keepdim=True)
+                # a zero matrix has no direction: its second term is nothing, as in the kernel
+                along = torch.where(r > 0, dot / (torch.where(r > 0, r, 1.0) * (r + ctx.eps) ** 2), 0.0)
+                g = g + (dxv / (r + ctx.eps) - v * along).view_as(g)
+            rows = (m.numel(), -1)
+            return (g, (m[:, None] * g.reshape(rows)).view_as(z) if need_z else None,
+                    (g.reshape(rows) * z.reshape(rows)).sum(1) if need_m else None, None, None)
         da, dz, dm = cuda_ext(z).momentum_normalize_bwd(z_new, z, m, sumsq, dz_new, dx, ctx.eps, need_z, need_m)
         return da, dz if need_z else None, dm if need_m else None, None, None
 
