@@ -79,6 +79,57 @@ def test_momentum_and_normalisation(bsz, e, r, rows, d):
             assert _rel(x, y) < 3e-2
 
 
+def _odd(t, offset):
+    """The same values as a contiguous view that starts ``offset`` elements into a buffer."""
+    view = t.new_empty(t.numel() + offset)[offset:].view(t.shape)
+    return view.copy_(t)
+
+
+# Each output alone and both, gradients that start on and off a 16-byte boundary (the backward of a concatenation hands
+# out the latter); expectation from the formulas in 64 bits.
+@pytest.mark.parametrize("use_z,use_x", [(True, True), (True, False), (False, True)])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_momentum_gradients_at_any_alignment(use_z, use_x, offset):
+    ext = load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(offset)
+    bsz, e, r, d, rows = 2, 3, 256, 128, 128
+    n = bsz * e * r // rows
+    a, z, gz = (torch.randn(bsz, e, r, d, generator=gen, device=DEV) for _ in range(3))
+    m, gx = torch.rand(bsz, generator=gen, device=DEV), torch.randn(a.shape, generator=gen, device=DEV).bfloat16()
+    z_new, x, sumsq = ext.momentum_normalize_fwd(a, z, m, n, 1e-7)
+    da, dz, dm = ext.momentum_normalize_bwd(z_new, z, m, sumsq, _odd(gz, offset) if use_z else None,
+                                            _odd(gx, offset) if use_x else None, 1e-7, True, True)
+    t = [v.double().requires_grad_() for v in (a, z, m)]
+    zn = t[0] + t[2].view(-1, 1, 1, 1) * t[1]
+    xn = (zn.view(n, -1) / (zn.view(n, -1).norm(dim=1, keepdim=True) + 1e-7)).view(a.shape)
+    outs, cots = zip(*([(zn, gz.double())] * use_z + [(xn, gx.double())] * use_x))
+    assert _rel(z_new, zn) < 1e-6 and _rel(sumsq, zn.view(n, -1).pow(2).sum(1)) < 1e-5
+    assert _rel(x, xn) < 2 ** -8                                 # bf16
+    for got, want in zip((da, dz, dm), torch.autograd.grad(outs, t, cots)):
+        assert _rel(got, want) < 1e-5                            # fp32 products and sums of 1e5 of them
+
+
+def test_momentum_gradients_refuse_other_sizes():
+    ext = load(required=True)
+    a, m = torch.randn(1, 1, 128, 128, device=DEV), torch.rand(1, device=DEV)
+    z_new, _, sumsq = ext.momentum_normalize_fwd(a, a, m, 1, 1e-7)
+    for bad in ((a[:, :, :64], None), (None, a[:, :, :64].bfloat16())):
+        with pytest.raises(RuntimeError):
+            ext.momentum_normalize_bwd(z_new, a, m, sumsq, *bad, 1e-7, True, True)
+    with pytest.raises(RuntimeError):
+        ext.momentum_normalize_bwd(z_new, a[:, :, :64], m, sumsq, a, None, 1e-7, True, True)
+
+
+def test_momentum_gradient_through_a_concatenation():
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    a, z = (torch.randn(1, 2, 256, 128, generator=gen, device=DEV).requires_grad_() for _ in range(2))
+    m, w = torch.rand(1, 1, 1, 1, generator=gen, device=DEV), torch.randn(1 + a.numel(), generator=gen, device=DEV)
+    z_new, _ = ops.momentum_newton_schulz(a, z, m, 256)
+    da, dz = torch.autograd.grad((torch.cat([a.new_zeros(1), z_new.flatten()]) * w).sum(), (a, z))
+    assert torch.equal(da.flatten(), w[1:]) and _rel(dz.flatten(), w[1:].double() * m.double().item()) < 1e-6
+
+
 @pytest.mark.parametrize("d", [4, 512, 516, 1536, 2048])
 @pytest.mark.parametrize("renorm", ["restore", "unit", "none"])
 @pytest.mark.parametrize("rows", [1, 3, 700])

@@ -20,6 +20,7 @@
 #include <torch/extension.h>
 
 #include "common.cuh"
+#include "operand.h"
 
 namespace uttt {
 
@@ -553,13 +554,24 @@ std::vector<at::Tensor> momentum_normalize_bwd(at::Tensor z_new, at::Tensor z, a
                                                bool need_dz, bool need_dm) {
   c10::cuda::CUDAGuard guard(z_new.device());
   const int64_t matrices = sumsq.numel();
+  TORCH_CHECK(matrices > 0 && sumsq.scalar_type() == at::kFloat && sumsq.is_contiguous());
+  z_new = dense16(z_new);
+  z = dense16(z);
+  check_bank(z_new, matrices);
+  check_bank(z, matrices);
+  TORCH_CHECK(z.numel() == z_new.numel() && m.scalar_type() == at::kFloat && m.is_contiguous() && m.numel() > 0 &&
+              matrices % m.numel() == 0 && matrices <= 65535);
   const long long per = z_new.numel() / matrices;
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   const dim3 grid = frob_grid(per, (int)matrices);
   at::Tensor gz, gx, dot;
-  if (dz_new.has_value() && dz_new->defined()) gz = dz_new->to(at::kFloat).contiguous();
+  if (dz_new.has_value() && dz_new->defined()) {
+    gz = dense16(dz_new->to(at::kFloat));
+    TORCH_CHECK(gz.numel() == z_new.numel() && gz.device() == z_new.device());
+  }
   if (dx.has_value() && dx->defined()) {
-    gx = dx->to(at::kBFloat16).contiguous();
+    gx = dense16(dx->to(at::kBFloat16));
+    TORCH_CHECK(gx.numel() == z_new.numel() && gx.device() == z_new.device());
     dot = at::zeros({matrices}, sumsq.options());
     frob_partial_kernel<float><<<grid, 256, 0, stream>>>(z_new.data_ptr<float>(),
                                                          reinterpret_cast<const __nv_bfloat16*>(gx.data_ptr()),
