@@ -120,6 +120,18 @@ def test_momentum_gradients_refuse_other_sizes():
         ext.momentum_normalize_bwd(z_new, a[:, :, :64], m, sumsq, a, None, 1e-7, True, True)
 
 
+def test_momentum_gradients_repeat_bit_for_bit():
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    t = [torch.randn(2, 4, 768, 384, generator=gen, device=DEV).requires_grad_() for _ in range(2)]
+    t.append(torch.rand(2, 1, 1, 1, generator=gen, device=DEV).requires_grad_())
+    z_new, _ = ops.momentum_newton_schulz(*t, 384)
+    g = torch.randn(z_new.shape, generator=gen, device=DEV)
+    first = torch.autograd.grad(z_new, t, g, retain_graph=True)
+    for _ in range(8):
+        assert all(torch.equal(x, y) for x, y in zip(torch.autograd.grad(z_new, t, g, retain_graph=True), first))
+
+
 def test_momentum_gradient_through_a_concatenation():
     load(required=True)
     gen = torch.Generator(device=DEV).manual_seed(9)

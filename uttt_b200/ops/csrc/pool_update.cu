@@ -467,7 +467,8 @@ __global__ void __launch_bounds__(256) momentum_sumsq_kernel(const float* __rest
   }
 }
 
-// dx, dz_new, dz and dm may be absent; dm[b] collects <g, z> of matrix b
+// dx, dz_new, dz and dm may be absent; dm[b, chunk] = the block's share of <g, z> of matrix b, so that the sum over the
+// blocks has one order
 __global__ void __launch_bounds__(256) momentum_bwd_kernel(const float* __restrict__ z_new, const float* __restrict__ z,
                                                            const float* __restrict__ m, const __nv_bfloat16* __restrict__ dx,
                                                            const float* __restrict__ dz_new, const float* __restrict__ sumsq,
@@ -516,7 +517,7 @@ __global__ void __launch_bounds__(256) momentum_bwd_kernel(const float* __restri
   if (threadIdx.x == 0) {
     float s = 0.f;
     for (int i = 0; i < 8; ++i) s += red[i];
-    atomicAdd(dm + b, s);
+    dm[b * gridDim.x + blockIdx.x] = s;
   }
 }
 
@@ -580,7 +581,7 @@ std::vector<at::Tensor> momentum_normalize_bwd(at::Tensor z_new, at::Tensor z, a
   }
   auto da = at::empty_like(z_new);
   auto dz = need_dz ? at::empty_like(z) : at::empty({0}, z.options());
-  auto dm = need_dm ? at::zeros({matrices}, m.options()) : at::empty({0}, m.options());
+  auto dm = at::empty({need_dm ? matrices : 0, (int64_t)grid.x}, m.options());
   momentum_bwd_kernel<<<grid, 256, 0, stream>>>(
       z_new.data_ptr<float>(), z.data_ptr<float>(), m.data_ptr<float>(),
       gx.defined() ? reinterpret_cast<const __nv_bfloat16*>(gx.data_ptr()) : nullptr,
@@ -589,8 +590,7 @@ std::vector<at::Tensor> momentum_normalize_bwd(at::Tensor z_new, at::Tensor z, a
       per, (int)(matrices / m.numel()));
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   count_launch();
-  if (need_dm) dm = dm.view({m.numel(), -1}).sum(1);
-  return {da, dz, dm};
+  return {da, dz, need_dm ? dm.view({m.numel(), -1}).sum(1) : dm};
 }
 
 }  // namespace uttt
