@@ -54,6 +54,43 @@ def test_attention_tile_edges(b, h, lq, lk, hd, window, causal, scale):
             assert _rel(got, ref_) < 1e-2, (name, _rel(got, ref_))
 
 
+# 364 keys, the queries on the last 300: query tile 0 sees keys 0..191 (from 1 with the window), key 200 is seen by query 136 on;
+# query 10 sees keys 11..74, so the keys from 128 on see nothing of it.
+@pytest.mark.parametrize("hd", [64, 96, 128])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("window,causal", [(64, True), (None, True)])
+def test_attention_masked_values_that_are_not_finite(hd, value, window, causal):
+    """A NaN or an infinity stays in the tiles that see it: the products skip the masked groups of 16."""
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(hd)
+    base = [torch.randn(1, n, 2, hd, generator=gen, device=DEV).bfloat16() for n in (300, 364, 364, 300)]      # q, k, v, do
+
+    def run(which, row):
+        t = [x.clone() for x in base]
+        if which is not None:
+            t[which][:, row] = value
+        leaves = [x.requires_grad_() for x in t[:3]]
+        out = ops.swa_attention(*leaves, window, causal=causal)
+        res = [out.detach(), *torch.autograd.grad(out, leaves, t[3])]
+        torch.cuda.synchronize()
+        _status_ok()
+        return res
+
+    clean = run(None, 0)
+    for which in (1, 2):                                         # a key, a value: what its queries' tile does not reach
+        got = run(which, 200)
+        for i in (0, 1):
+            assert bool(got[i][:, :128].isfinite().all())
+            assert _rel(got[i][:, :128], clean[i][:, :128]) < 1e-3       # dQ adds in any order before it is rounded to bf16
+            assert not bool(got[i][:, 199].isfinite().all())             # and the queries that see it are told
+    if window is not None:
+        for which in (0, 3):                                     # a query, a gradient
+            got = run(which, 10)
+            for i in (2, 3):
+                assert torch.equal(got[i][:, 128:], clean[i][:, 128:])
+                assert not bool(got[i][:, 74].isfinite().all())
+
+
 @pytest.mark.parametrize("bsz,e,r,rows,d", [(1, 1, 256, 128, 128), (3, 2, 384, 384, 128), (2, 3, 512, 256, 384)])
 def test_momentum_and_normalisation(bsz, e, r, rows, d):
     """Values and gradients against the two separate operations, with each output used alone and both together."""

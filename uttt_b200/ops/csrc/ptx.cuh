@@ -92,6 +92,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* status, int code) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
 }
+// The k-steps lo..hi of a product of N, f(step, first of them); all of them, the usual case, unrolled: with a condition at
+// every step of the unrolled form attention took 6 to 11 % longer.
+template <int N, typename F>
+__device__ __forceinline__ void mma_groups(int lo, int hi, F&& f) {
+  if (lo == 0 && hi == N - 1) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) f(k, k == 0);
+  } else {
+#pragma unroll 1
+    for (int k = lo; k <= hi; ++k) f(k, k == lo);
+  }
+}
 template <typename T>
 __device__ __forceinline__ T warp_uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
 

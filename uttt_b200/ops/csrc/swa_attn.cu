@@ -176,6 +176,15 @@ __global__ void __launch_bounds__(kThreads, 1) swa_fwd_kernel(const __grid_const
       // S_j overwrites P_{j-1}: the product that reads P_{j-1} was issued before it by this thread, and the tensor core
       // runs them in order.  For the same reason "S_j is complete" says that O has received P_{j-1} V_{j-1}.
       const bool leader = ptx::elect_one();
+      // P is zero where it is masked, but zero times a NaN or an infinity in V is not: the product leaves out the groups
+      // of 16 keys that no query of the tile sees.
+      int key_lo[2], key_hi[2];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int q0 = q00 + s * kQ;
+        key_lo[s] = p.causal && p.window > 0 ? max(0, shift + q0 - p.window + 1) : 0;
+        key_hi[s] = p.causal ? min(p.lk - 1, shift + q0 + kQ - 1) : p.lk - 1;
+      }
       for (int j = 0; j <= nt && ok; ++j) {
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
@@ -187,11 +196,12 @@ __global__ void __launch_bounds__(kThreads, 1) swa_fwd_kernel(const __grid_const
                  ptx::warp_wait(v_full(st), ((j - 1) / ST) & 1, p.status, 14);
             if (!ok) break;
             ptx::tc_fence_after_sync();
-#pragma unroll
-            for (int k = 0; k < kKV / 16; ++k) {
+            const int key0 = (t0 + j - 1) * kKV;
+            const int klo = max(0, key_lo[s] - key0) >> 4, khi = min(kKV - 1, key_hi[s] - key0) >> 4;
+            ptx::mma_groups<kKV / 16>(klo, khi, [&](int k, bool start) {
               const uint64_t db = ptx::make_smem_desc(v_smem(st) + k * 2048, kSlabBytes, 1024);   // V_j (N-major slabs)
-              if (leader) ptx::mma_bf16_ts(tmem_o(s), tmem_s(s) + k * 8, db, idesc_o, (j - 1 > first || k > 0) ? 1u : 0u);
-            }
+              if (leader) ptx::mma_bf16_ts(tmem_o(s), tmem_s(s) + k * 8, db, idesc_o, (j - 1 > first || !start) ? 1u : 0u);
+            });
             if (leader && j - 1 == last) ptx::mma_commit(o_done(s));
           }
           if (j >= first && j <= last) {

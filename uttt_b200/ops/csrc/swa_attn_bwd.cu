@@ -261,34 +261,38 @@ __global__ void __launch_bounds__(kThreads, 1) swa_bwd_kernel(const __grid_const
         return true;
       };
       ok = ptx::warp_wait(kv_full, 0, p.status, 35) && issue_s(0) && issue_dp(0);
+      // P and dS are zero where they are masked (dS is NaN there when dP is), but zero times a NaN or an infinity is not:
+      // the sums over queries leave out the groups of 16 that see no key of this block, the sum over keys the groups that
+      // no query of the tile sees.
       for (int j = 0; j < nq && ok; ++j) {
-        const int s = j & 1;
+        const int s = j & 1, q0 = (t0 + j) * kT;
+        const int qlo = max(0, first_q - q0) >> 4, qhi = min(kT - 1, last_q - q0) >> 4;
+        const int key_lo = p.causal && p.window > 0 ? shift + q0 - p.window + 1 : 0;
+        const int key_hi = p.causal ? min(p.lk - 1, shift + q0 + kT - 1) : p.lk - 1;
+        const int klo = max(0, key_lo - k0) >> 4, khi = min(kT - 1, key_hi - k0) >> 4;
         ok = ptx::warp_wait(p_ready, j & 1, p.status, 36);
         if (!ok) break;
         ptx::tc_fence_after_sync();
-#pragma unroll
-        for (int k = 0; k < kT / 16; ++k) {
+        ptx::mma_groups<kT / 16>(qlo, qhi, [&](int k, bool start) {
           const uint64_t db = ptx::make_smem_desc(do_smem + k * 2048, kSlab, 1024);         // dO (N-major slabs)
-          if (leader) ptx::mma_bf16_ts(tmem_dv, tmem_s + (k >> 2) * 64 + (k & 3) * 8, db, idesc_acc, (j > 0 || k > 0) ? 1u : 0u);
-        }
+          if (leader) ptx::mma_bf16_ts(tmem_dv, tmem_s + (k >> 2) * 64 + (k & 3) * 8, db, idesc_acc, (j > 0 || !start) ? 1u : 0u);
+        });
         if (leader) ptx::mma_commit(do_empty);
         if (j + 1 < nq) ok = issue_s(j + 1);
         ok = ok && ptx::warp_wait(ds_ready, j & 1, p.status, 37);
         if (!ok) break;
         ptx::tc_fence_after_sync();
-#pragma unroll
-        for (int k = 0; k < kT / 16; ++k) {
+        ptx::mma_groups<kT / 16>(klo, khi, [&](int k, bool start) {
           const uint64_t da = ptx::make_smem_desc(ds_smem + k * 2048, kSlab, 1024);          // dS (M-major: queries)
           const uint64_t db = ptx::make_smem_desc(k_smem + k * 2048, kSlab, 1024);           // K (N-major slabs)
-          if (leader) ptx::mma_bf16_ss(tmem_dp, da, db, idesc_dq, k > 0 ? 1u : 0u);
-        }
+          if (leader) ptx::mma_bf16_ss(tmem_dp, da, db, idesc_dq, start ? 0u : 1u);
+        });
         if (leader) ptx::mma_commit(dq_done);
-#pragma unroll
-        for (int k = 0; k < kT / 16; ++k) {
+        ptx::mma_groups<kT / 16>(qlo, qhi, [&](int k, bool start) {
           const uint64_t da = ptx::make_smem_desc(ds_smem + (k >> 2) * kSlab + (k & 3) * 32, 16, 1024);   // dS^T
           const uint64_t db = ptx::make_smem_desc(q_smem(s) + k * 2048, kSlab, 1024);        // Q (N-major slabs)
-          if (leader) ptx::mma_bf16_ss(tmem_dk, da, db, idesc_acc, (j > 0 || k > 0) ? 1u : 0u);
-        }
+          if (leader) ptx::mma_bf16_ss(tmem_dk, da, db, idesc_acc, (j > 0 || !start) ? 1u : 0u);
+        });
         if (leader) ptx::mma_commit(q_empty(s));
         if (j + 1 < nq) ok = ptx::warp_wait(dq_free, j & 1, p.status, 38) && issue_dp(j + 1);
       }
