@@ -91,6 +91,31 @@ def test_attention_masked_values_that_are_not_finite(hd, value, window, causal):
                 assert not bool(got[i][:, 74].isfinite().all())
 
 
+# Windows shorter and longer than a tile, bands that end at the last launch's tiles, no window, no mask.
+@pytest.mark.parametrize("lq,lk,window,causal", [(1100, 2100, 1, True), (1100, 2100, 300, True), (1280, 1280, 131, True),
+                                                 (1100, 2100, None, True), (700, 900, None, False), (100, 100, 64, True)])
+def test_attention_gradients_repeat_bit_for_bit_when_asked(lq, lk, window, causal):
+    """torch.use_deterministic_algorithms gives the sums of dQ an order; the values stay what they are without it."""
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(lq)
+    q, k, v, do = (torch.randn(2, n, 8, 64, generator=gen, device=DEV).bfloat16() for n in (lq, lk, lk, lq))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    out = ops.swa_attention(*leaves, window, causal=causal)
+    grads = lambda: torch.autograd.grad(out, leaves, do, retain_graph=True)
+    plain = grads()
+    torch.use_deterministic_algorithms(True, warn_only=True)
+    try:
+        first = grads()
+        for _ in range(6):
+            assert all(torch.equal(x, y) for x, y in zip(grads(), first))
+    finally:
+        torch.use_deterministic_algorithms(False)
+    _status_ok()
+    assert torch.equal(first[1], plain[1]) and torch.equal(first[2], plain[2])
+    # fp32 sums in another order, then rounded to bf16: a few elements move by one unit
+    assert _rel(first[0], plain[0]) < 1e-3 or float(plain[0].float().abs().max()) < 2e-2
+
+
 @pytest.mark.parametrize("bsz,e,r,rows,d", [(1, 1, 256, 128, 128), (3, 2, 384, 384, 128), (2, 3, 512, 256, 384)])
 def test_momentum_and_normalisation(bsz, e, r, rows, d):
     """Values and gradients against the two separate operations, with each output used alone and both together."""

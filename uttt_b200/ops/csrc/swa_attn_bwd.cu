@@ -19,8 +19,9 @@
 //   swa_bwd_dq_out_kernel  fp32 dQ sums -> bf16, scaled
 // S, P and dS are formed once for all three gradients: five products and one exponential per element, where separate
 // dK/dV and dQ kernels needed seven and two.  The price is the addition of dQ in L2 (48 KB per tile at 96), in no fixed
-// order, in fp32.  Bound by the hand-overs between the products and the warps.  Measured with its preparation and
-// conversion: 785 -> 459 us at 4 x 16 heads x 96, 2048 queries on 4096 keys, window 2048.
+// order, to fp32 sums of b * h * ceil(lq, 128) * hd that are allocated and cleared on every call (50 MB at the size below).  Bound by the hand-overs between the products and the warps.  Measured with its preparation and
+// conversion: 785 -> 459 us at 4 x 16 heads x 96, 2048 queries on 4096 keys, window 2048.  With deterministic algorithms
+// asked for, the additions have an order: see launch_bwd.
 // Warps: 0-7 P and dS (two per TMEM lane quarter, each owning half of the 128 columns of a tile), 8-11 dQ,
 // 12 TMA producer lane, 13 MMA issuer lane.  Every wait is bounded (ptx::mbar_wait).
 #include <ATen/ATen.h>
@@ -42,6 +43,7 @@ struct SwaBwdParams {
   int lq, lk, heads, lq_pad;
   int window;          // 0 = unlimited
   int causal;
+  int kt_first, kt_step;   // the launch's key tiles: kt_first + blockIdx.x * kt_step
   float scale, scale_log2;
   const float* nlse2;  // [b, h, lq_pad]  -lse * log2(e); -inf on padding rows
   const float* ndsum;  // [b, h, lq_pad]  -D; 0 on padding rows
@@ -142,8 +144,8 @@ __global__ void __launch_bounds__(kThreads, 1) swa_bwd_kernel(const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + C::kBars + 128);
 
   const int warp = ptx::warp_uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
-  const int kt = blockIdx.x, head = blockIdx.y, batch = blockIdx.z;
-  const int k0 = kt * kT;
+  const int head = blockIdx.y, batch = blockIdx.z;
+  const int k0 = (p.kt_first + (int)blockIdx.x * p.kt_step) * kT;
   const int shift = p.lk - p.lq;
   // queries that can see any key of [k0, k0 + 127]
   int first_q = 0, last_q = p.lq - 1;
@@ -480,7 +482,7 @@ __global__ void __launch_bounds__(256) swa_bwd_dq_out_kernel(const float* __rest
 // ------------------------------------------------------------------------------------ host
 template <int HD>
 static void launch_bwd(const at::Tensor& o, const at::Tensor& dout, const at::Tensor& lse, const CUtensorMap& tq,
-                       const CUtensorMap& tdo, const CUtensorMap& tk, const CUtensorMap& tv, const SwaBwdParams& p,
+                       const CUtensorMap& tdo, const CUtensorMap& tk, const CUtensorMap& tv, SwaBwdParams p,
                        float* nlse2, float* ndsum, __nv_bfloat16* dq, int b, cudaStream_t stream) {
   const int total = b * p.heads * p.lq_pad;
   swa_bwd_prep_kernel<HD><<<(total + 31) / 32, 256, 0, stream>>>(
@@ -489,8 +491,21 @@ static void launch_bwd(const at::Tensor& o, const at::Tensor& dout, const at::Te
   C10_CUDA_KERNEL_LAUNCH_CHECK();
   auto kernel = swa_bwd_kernel<HD>;
   C10_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<HD>::kSmem));
-  kernel<<<dim3((p.lk + kT - 1) / kT, p.heads, b), kThreads, BwdCfg<HD>::kSmem, stream>>>(tq, tdo, tk, tv, p);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
+  // Under torch.use_deterministic_algorithms a launch takes only key tiles whose bands share no query tile, every
+  // kt_step-th one: it adds at most once to any sum of dQ, and the launches follow one another.  A band of 128 keys and a
+  // window covers fewer than (window + 253) / 128 + 1 query tiles.  4 x 16 heads x 96, 2048 queries on 4096 keys,
+  // window 2048: 968 us for the whole backward, against 528 with all key tiles in one launch (the two kernels that this one
+  // replaced, which needed no such order, 785).
+  const int tiles = (p.lk + kT - 1) / kT;
+  p.kt_step = 1;
+  if (at::globalContext().deterministicAlgorithms())
+    p.kt_step = p.causal && p.window > 0 ? (int)std::min<long long>(tiles, ((long long)p.window + 253) / kT + 1) : tiles;
+  for (p.kt_first = 0; p.kt_first < p.kt_step; ++p.kt_first) {
+    const int blocks = (tiles - p.kt_first + p.kt_step - 1) / p.kt_step;
+    kernel<<<dim3(blocks, p.heads, b), kThreads, BwdCfg<HD>::kSmem, stream>>>(tq, tdo, tk, tv, p);
+    C10_CUDA_KERNEL_LAUNCH_CHECK();
+    count_launch();
+  }
   swa_bwd_dq_out_kernel<HD><<<p.lq_pad / 64 * p.heads * b, 256, 0, stream>>>(p.dq_sum, dq, p.scale, p.lq, p.lq_pad,
                                                                                   p.heads);
   C10_CUDA_KERNEL_LAUNCH_CHECK();
@@ -537,9 +552,7 @@ std::vector<at::Tensor> swa_bwd(at::Tensor dout, at::Tensor q, at::Tensor k, at:
   if (hd == 64) launch_bwd<64>(o, dout, lse, tq, tdo, tk, tv, p, nlse2, ndsum, dqp, b, stream);
   else if (hd == 96) launch_bwd<96>(o, dout, lse, tq, tdo, tk, tv, p, nlse2, ndsum, dqp, b, stream);
   else launch_bwd<128>(o, dout, lse, tq, tdo, tk, tv, p, nlse2, ndsum, dqp, b, stream);
-  count_launch();
-  count_launch();
-  count_launch();
+  count_launch(2);
   return {dq, dk, dv};
 }
 

@@ -149,8 +149,10 @@ def main(job: Optional[JobConfig] = None) -> TrainState:
     if job.job.print_args and rank == 0:
         print(json.dumps(job.to_dict(), indent=1, default=str))
     if job.training.deterministic:
-        # same seed, same reduction order: bit-identical reruns (the kernels of this framework use fixed
-        # reduction orders except the embedding-gradient scatter, which uses fp32 reductions in memory)
+        # Same seed, and one order of sums in the library's operations and in attention (whose dQ is otherwise summed in
+        # arrival order).  These kernels still add in arrival order, so reruns agree closely and not to the bit:
+        # the embedding-gradient scatter, the router's balance sums, d(scale) and d(shift) of the memory preprocessing,
+        # the matrix norms of the orthogonalisation, the loss and the gradient norm.
         os.environ.setdefault("CUBLAS_WORKSPACE_CONFIG", ":4096:8")
         torch.use_deterministic_algorithms(True, warn_only=True)
         torch.backends.cudnn.deterministic, torch.backends.cudnn.benchmark = True, False
