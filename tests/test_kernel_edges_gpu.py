@@ -312,3 +312,22 @@ def test_router_matches_double_precision(e, d, kind, bsz, n, topk):
     # fp32 logits: d 2^-24 of their size at most; __expf adds 2^-21 of its argument
     torch.testing.assert_close(w.view(bsz, n, topk).double(), probs.gather(-1, idx.long()) * 0.7, atol=2e-6, rtol=1e-4)
     torch.testing.assert_close(psum.double(), probs.sum(1), atol=1e-4, rtol=1e-4)
+
+
+# Both variants, both row types; a router off a 16-byte boundary goes to the general kernel.
+@pytest.mark.parametrize("e,d,dtype", [(16, 64, torch.bfloat16), (24, 128, torch.bfloat16), (16, 64, torch.float32)])
+@pytest.mark.parametrize("rows_off,router_off", [(1, 0), (0, 1), (3, 2)])
+def test_router_operands_at_any_alignment(e, d, dtype, rows_off, router_off):
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(e + d)
+    rows = torch.randn(2, 300, d, generator=gen, device=DEV).to(dtype)
+    router = torch.randn(e, d, generator=gen, device=DEV) * d ** -0.5
+    gw = torch.randn(600, 2, generator=gen, device=DEV)
+    res = []
+    for r, w in ((rows, router), (_odd(rows, rows_off), _odd(router, router_off))):
+        leaves = [r.requires_grad_(), w.requires_grad_()]
+        idx, wts, psum = ops.route_topk(*leaves, None, 2)
+        res.append((wts.detach(), psum.detach(), *torch.autograd.grad(wts, leaves, gw)))
+    _status_ok()
+    for got, want in zip(res[1], res[0]):
+        assert _rel(got, want) < (1e-5 if got.dtype == torch.float32 else 2 ** -8)

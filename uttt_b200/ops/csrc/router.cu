@@ -23,6 +23,7 @@
 #include <torch/extension.h>
 
 #include "common.cuh"
+#include "operand.h"
 #include "ptx.cuh"
 #include "tc_gemm.cuh"
 
@@ -739,6 +740,7 @@ std::vector<at::Tensor> router_fwd(at::Tensor rows, at::Tensor router, c10::opti
   TORCH_CHECK(rows.dim() == 2 && rows.is_contiguous() && router.is_contiguous() && router.scalar_type() == at::kFloat);
   const int R = rows.size(0), D = rows.size(1), E = router.size(0);
   TORCH_CHECK(router.size(1) == D && router_supported(D, E, topk) && R % rows_per_batch == 0);
+  rows = dense16(rows);                           // both variants fetch rows 16 bytes at a time
   const float* bp = nullptr;
   at::Tensor bc;
   if (bias.has_value() && bias->defined()) {
@@ -755,11 +757,11 @@ std::vector<at::Tensor> router_fwd(at::Tensor rows, at::Tensor router, c10::opti
   auto logits = mode != 0 ? at::empty({R, E}, opts.dtype(at::kFloat)) : at::empty({0}, opts.dtype(at::kFloat));
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   // Tensor cores need whole 64-column slabs, an expert count that is an MMA width, room for the three router parts, and an
-  // accumulator per slab and tile.
+  // accumulator per slab and tile; the general kernel reads the router one value at a time, from any address.
   const int tc_smem = router_tc_smem(D, E);
   const int slab_cols = E <= 16 ? 16 : E <= 32 ? 32 : 64;
   if (rows.scalar_type() == at::kBFloat16 && D % 64 == 0 && E % 16 == 0 && tc_smem <= 227 * 1024 - 64 && D / 64 * slab_cols <= 256 && R > 0 &&
-      ((uintptr_t)rows.data_ptr() & 15) == 0 && ((uintptr_t)router.data_ptr() & 15) == 0) {
+      ((uintptr_t)router.data_ptr() & 15) == 0) {
     RouterTcParams tp{router.data_ptr<float>(), bp, R, D, (int)topk, (int)rows_per_batch, (float)alpha,
                       bias_in_logits ? 1 : 0, renorm ? 1 : 0, (int)mode, (float)rscale, (float)norm_eps,
                       idx.data_ptr<int>(), w.data_ptr<float>(), probs.data_ptr<float>(), psum.data_ptr<float>(),
@@ -853,6 +855,7 @@ std::vector<at::Tensor> router_bwd(at::Tensor rows, at::Tensor router, at::Tenso
   c10::cuda::CUDAGuard guard(rows.device());
   const int R = rows.size(0), D = rows.size(1), E = router.size(0), topk = idx.size(1);
   TORCH_CHECK(router_supported(D, E, topk) && probs.is_contiguous() && idx.is_contiguous() && rows.is_contiguous());
+  rows = dense16(rows);
   at::Tensor dwc, dpc;
   const float *dwp = nullptr, *dpp = nullptr;
   if (dweights.has_value() && dweights->defined()) {
