@@ -5,6 +5,7 @@ import torch
 import torch.nn.functional as F
 
 from uttt_b200 import ops
+from uttt_b200.ops import functional
 from uttt_b200.ops import reference as ref
 from uttt_b200.ops._ext import load
 
@@ -331,3 +332,50 @@ def test_router_operands_at_any_alignment(e, d, dtype, rows_off, router_off):
     _status_ok()
     for got, want in zip(res[1], res[0]):
         assert _rel(got, want) < (1e-5 if got.dtype == torch.float32 else 2 ** -8)
+
+
+def _alignment_cases(gen):
+    """name -> (function of the leaves, leaves): every op whose kernel moves 16 bytes at a time."""
+    rnd = lambda *shape: torch.randn(*shape, generator=gen, device=DEV)
+    plan = ops.build_group_plan(torch.randint(0, 3, (1, 37, 2), generator=gen, device=DEV), 3)
+    rows, ids = plan.rows_padded, torch.randint(0, 50, (2, 9), generator=gen, device=DEV)
+    weight = rnd(37, 2).abs()
+    return {
+        "rms_norm": (lambda x, w: ops.rms_norm(x, w), (rnd(37, 64), rnd(64))),
+        "rms_norm_gated": (lambda x, w, g: ops.rms_norm_gated(x, w, g), (rnd(37, 64), rnd(64), rnd(37))),
+        "add_rms_norm": (lambda x, y, w: torch.cat(ops.add_rms_norm(x, y, w)), (rnd(37, 64), rnd(37, 64), rnd(64))),
+        "rope": (lambda x: ops.rope(x, 3, 1e4), (rnd(2, 9, 2, 32),)),
+        "fw_qk_prep": (lambda x, a, b: ops.fw_qk_prep(x, a, b, 2, 32, 1e4, 5, True, "l2"), (rnd(2, 9, 64), rnd(64), rnd(64))),
+        "swiglu": (lambda y: ops.swiglu(y), (rnd(37, 64),)),
+        "fw_write_pointwise": (lambda y, d, r: torch.cat(functional.fw_write_pointwise(y, d, r), 1), (rnd(37, 64), rnd(37, 32), rnd(37, 3))),
+        "permute": (lambda x: ops.permute_rows(x, plan)[plan.dest.flatten()], (rnd(37, 64),)),
+        # (its gradient is defined for the rows that hold a copy)
+        "unpermute": (lambda y: ops.unpermute_rows(y, plan, weight), (rnd(rows, 64),), plan.dest.flatten()),
+        "embedding": (lambda t: ops.embedding(ids, t), (rnd(50, 64),)),
+        "pool_step": (lambda m, d: ops.pool_step(m, d, 0.3)[0], (rnd(37, 64), rnd(37, 64))),
+        "normalise": (lambda g: functional._FrobNormalize.apply(g, 1e-7), (rnd(2, 8, 16),)),
+    }
+
+
+@pytest.mark.parametrize("name", [
+    "rms_norm", "rms_norm_gated", "add_rms_norm", "rope", "fw_qk_prep", "swiglu", "fw_write_pointwise", "permute",
+    "unpermute", "embedding", "pool_step", "normalise"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_operands_at_any_alignment(name, dtype):
+    """Values and gradients do not depend on where a contiguous operand or gradient starts."""
+    load(required=True)
+    gen = torch.Generator(device=DEV).manual_seed(7)
+    fn, leaves, *defined = _alignment_cases(gen)[name]
+    if name != "pool_step":                                      # fp32 masters only
+        leaves = [t.to(dtype) for t in leaves]
+    res, gout = [], None
+    for offset in (0, 1, 3):
+        t = [_odd(x, offset).requires_grad_() for x in leaves]
+        out = fn(*t)
+        gout = torch.randn(out.shape, generator=gen, device=DEV).to(out.dtype) if gout is None else gout
+        grads = torch.autograd.grad(out, t, _odd(gout, offset))
+        res.append((out.detach(), *(g[defined[0]] if defined else g for g in grads)))
+    torch.cuda.synchronize()
+    for other in res[1:]:
+        for a, b in zip(other, res[0]):
+            assert _rel(a, b) < 1e-6 or torch.equal(a, b)        # the sums over rows may be added in another order

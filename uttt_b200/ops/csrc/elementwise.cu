@@ -9,6 +9,7 @@
 #include <torch/extension.h>
 
 #include "common.cuh"
+#include "operand.h"
 
 namespace uttt {
 
@@ -261,16 +262,17 @@ static std::vector<at::Tensor> rms_norm_fwd_impl(at::Tensor x, c10::optional<at:
   c10::cuda::CUDAGuard guard(x.device());
   int rows = x.size(0), d = x.size(1);
   TORCH_CHECK(x.is_contiguous() && d % 8 == 0);
+  x = dense16(x);
   auto y = at::empty_like(x);
   at::Tensor addc, sum;
   if (add.has_value() && add->defined()) {
     TORCH_CHECK(add->sizes() == x.sizes() && add->scalar_type() == x.scalar_type() && add->is_contiguous());
-    addc = *add;
+    addc = dense16(*add);
     sum = at::empty_like(x);
   }
   auto rstd = at::empty({rows}, x.options().dtype(at::kFloat));
   at::Tensor wc;
-  if (w.has_value() && w->defined()) wc = w->to(x.scalar_type()).contiguous();
+  if (w.has_value() && w->defined()) wc = dense16(w->to(x.scalar_type()));
   at::Tensor sc;
   if (row_scale.has_value() && row_scale->defined()) {
     sc = row_scale->to(x.scalar_type()).contiguous();
@@ -309,8 +311,10 @@ static std::vector<at::Tensor> rms_norm_bwd_impl(at::Tensor dy, at::Tensor x, c1
   at::Tensor dresc;
   if (dres.has_value() && dres->defined()) {
     TORCH_CHECK(dres->sizes() == x.sizes() && dres->scalar_type() == x.scalar_type() && dres->is_contiguous());
-    dresc = *dres;
+    dresc = dense16(*dres);
   }
+  dy = dense16(dy);
+  x = dense16(x);
   int rows = x.size(0), d = x.size(1);
   TORCH_CHECK(d % 8 == 0 && d <= 8 * 32 * 16, "rms_norm_bwd: hidden size must be a multiple of 8 and <= 4096");
   auto dx = at::empty_like(x);
@@ -319,7 +323,7 @@ static std::vector<at::Tensor> rms_norm_bwd_impl(at::Tensor dy, at::Tensor x, c1
   const int per_block = 4 * (nv <= 4 ? 8 : nv <= 8 ? 4 : nv <= 16 ? 2 : 1);      // 4 warps, 32 / G rows each
   int blocks = std::max(1, std::min((rows + per_block - 1) / per_block, sm_count() * 4));
   if (w.has_value() && w->defined()) {
-    wc = w->to(x.scalar_type()).contiguous();
+    wc = dense16(w->to(x.scalar_type()));
     dw = at::empty({blocks, d}, x.options().dtype(at::kFloat));
   } else {
     dw = at::zeros({1}, x.options().dtype(at::kFloat));
@@ -417,6 +421,7 @@ __global__ void rope_vec_kernel(const T* __restrict__ x, T* __restrict__ y, cons
 at::Tensor rope_fwd(at::Tensor x, at::Tensor table, int64_t offset, bool inverse) {
   c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.dim() == 4 && x.is_contiguous());
+  x = dense16(x);
   int l = x.size(1), nh = x.size(2), hd = x.size(3);
   TORCH_CHECK(table.scalar_type() == at::kFloat && table.size(0) >= offset + l && table.size(1) == hd / 2);
   auto y = at::empty_like(x);
@@ -877,12 +882,13 @@ std::vector<at::Tensor> fw_qk_prep_fwd(at::Tensor x, c10::optional<at::Tensor> s
   c10::cuda::CUDAGuard guard(x.device());
   int rows = x.size(0), d = x.size(1);
   TORCH_CHECK(x.is_contiguous() && d % heads == 0);
+  x = dense16(x);
   auto y = at::empty_like(x);
   auto inv = at::empty({rows, heads}, x.options().dtype(at::kFloat));
   at::Tensor sc, sh;
   if (scale.has_value() && scale->defined()) {
-    sc = scale->to(x.scalar_type()).contiguous();
-    sh = shift->to(x.scalar_type()).contiguous();
+    sc = dense16(scale->to(x.scalar_type()));
+    sh = dense16(shift->to(x.scalar_type()));
   }
   size_t smem = (d + heads) * sizeof(float);
   if (qk_warp_form_ok(d, (int)heads, (int)rope_dim) && rows > 0) {
@@ -920,12 +926,14 @@ std::vector<at::Tensor> fw_qk_prep_bwd(at::Tensor dy, at::Tensor x, c10::optiona
   c10::cuda::CUDAGuard guard(x.device());
   int rows = x.size(0), d = x.size(1);
   TORCH_CHECK(d <= 256 * 16, "fw_qk_prep_bwd: hidden size must be <= 4096");
+  dy = dense16(dy);
+  x = dense16(x);
   auto dx = at::empty_like(x);
   at::Tensor sc, sh;
   bool has = scale.has_value() && scale->defined();
   if (has) {
-    sc = scale->to(x.scalar_type()).contiguous();
-    sh = shift->to(x.scalar_type()).contiguous();
+    sc = dense16(scale->to(x.scalar_type()));
+    sh = dense16(shift->to(x.scalar_type()));
   }
   auto dscale = at::zeros({has ? d : 1}, x.options().dtype(at::kFloat));
   auto dshift = at::zeros({has ? d : 1}, x.options().dtype(at::kFloat));
@@ -1046,6 +1054,7 @@ at::Tensor swiglu_fwd(at::Tensor y02) {
   size_t rows = y02.size(0);
   int inter = y02.size(1) / 2;
   TORCH_CHECK(y02.is_contiguous() && inter % 8 == 0);
+  y02 = dense16(y02);
   auto h = at::empty({(int64_t)rows, inter}, y02.options());
   UTTT_DISPATCH_FLOAT(y02, {
     swiglu_fwd_kernel<T><<<ew_blocks(rows * inter / 8), 256, 0, cur_stream()>>>(ptr<T>(y02), ptr<T>(h), rows, inter);
@@ -1058,6 +1067,8 @@ at::Tensor swiglu_bwd(at::Tensor dh, at::Tensor y02) {
   c10::cuda::CUDAGuard guard(y02.device());
   size_t rows = y02.size(0);
   int inter = y02.size(1) / 2;
+  dh = dense16(dh);
+  y02 = dense16(y02);
   auto out = at::empty_like(y02);
   UTTT_DISPATCH_FLOAT(y02, {
     swiglu_bwd_kernel<T><<<ew_blocks(rows * inter / 8), 256, 0, cur_stream()>>>(ptr<T>(dh), ptr<T>(y02), ptr<T>(out),
@@ -1071,6 +1082,9 @@ std::vector<at::Tensor> swiglu_bwd_bwd(at::Tensor G, at::Tensor dh, at::Tensor y
   c10::cuda::CUDAGuard guard(y02.device());
   size_t rows = y02.size(0);
   int inter = y02.size(1) / 2;
+  G = dense16(G);
+  dh = dense16(dh);
+  y02 = dense16(y02);
   auto d_dh = at::empty_like(dh);
   auto d_y02 = at::empty_like(y02);
   UTTT_DISPATCH_FLOAT(y02, {
@@ -1162,6 +1176,8 @@ std::vector<at::Tensor> fw_write_pw_fwd(at::Tensor y02, at::Tensor dh, at::Tenso
   size_t rows = y02.size(0);
   int inter = y02.size(1) / 2;
   TORCH_CHECK(lr.scalar_type() == at::kFloat && lr.size(0) == (int64_t)rows && lr.size(1) == 3 && inter % 8 == 0);
+  y02 = dense16(y02);
+  dh = dense16(dh);
   auto dy02 = at::empty_like(y02);
   auto hlr = at::empty_like(dh);
   UTTT_DISPATCH_FLOAT(y02, {
@@ -1176,6 +1192,10 @@ std::vector<at::Tensor> fw_write_pw_bwd(at::Tensor C, at::Tensor Ch, at::Tensor 
   c10::cuda::CUDAGuard guard(y02.device());
   size_t rows = y02.size(0);
   int inter = y02.size(1) / 2;
+  C = dense16(C);
+  Ch = dense16(Ch);
+  y02 = dense16(y02);
+  dh = dense16(dh);
   auto d_y02 = at::empty_like(y02);
   auto d_dh = at::empty_like(dh);
   auto d_lr = at::empty_like(lr);
@@ -1335,6 +1355,7 @@ at::Tensor permute_rows(at::Tensor x, at::Tensor dest, int64_t rows_padded, c10:
   int d = x.size(1);
   int k = dest.size(1);
   TORCH_CHECK(x.is_contiguous() && dest.is_contiguous() && dest.scalar_type() == at::kLong && d % 8 == 0);
+  x = dense16(x);
   size_t n = (size_t)dest.numel();
   const int per_block = copies_per_block(d);
   int blocks = (int)std::max<size_t>(1, std::min<size_t>((n + per_block - 1) / per_block, (size_t)sm_count() * 16));
@@ -1359,6 +1380,7 @@ at::Tensor unpermute_rows(at::Tensor y, at::Tensor dest, c10::optional<at::Tenso
   size_t rows = dest.size(0);
   int k = dest.size(1);
   TORCH_CHECK(y.is_contiguous() && d % 8 == 0);
+  y = dense16(y);
   at::Tensor wf;
   if (w.has_value() && w->defined()) wf = w->to(at::kFloat).contiguous();
   auto out = at::empty({(int64_t)rows, d}, y.options());
@@ -1381,6 +1403,8 @@ std::vector<at::Tensor> unpermute_rows_bwd(at::Tensor dout, at::Tensor y, at::Te
   int d = y.size(1);
   int k = dest.size(1);
   size_t n = (size_t)dest.numel();
+  dout = dense16(dout);
+  y = dense16(y);
   auto wf = w.to(at::kFloat).contiguous();
   const int per_block = copies_per_block(d);
   int blocks = (int)std::max<size_t>(1, std::min<size_t>((n + per_block - 1) / per_block, (size_t)sm_count() * 16));

@@ -14,6 +14,7 @@
 #include <torch/extension.h>
 
 #include "common.cuh"
+#include "operand.h"
 
 namespace uttt {
 
@@ -91,6 +92,7 @@ at::Tensor embedding_fwd(at::Tensor table, at::Tensor ids) {
   TORCH_CHECK(table.dim() == 2 && table.is_contiguous() && ids.scalar_type() == at::kLong);
   int d = table.size(1);
   TORCH_CHECK(d % 8 == 0, "embedding: hidden size must be a multiple of 8");
+  table = dense16(table);
   auto idc = ids.contiguous();
   size_t tokens = idc.numel();
   auto shape = idc.sizes().vec();
@@ -114,7 +116,7 @@ at::Tensor embedding_bwd(at::Tensor dy, at::Tensor ids, int64_t vocab) {
   c10::cuda::CUDAGuard guard(dy.device());
   int d = dy.size(-1);
   TORCH_CHECK(d % 8 == 0 && ids.scalar_type() == at::kLong);
-  auto dyc = dy.contiguous();
+  auto dyc = dense16(dy);
   auto idc = ids.contiguous();
   size_t tokens = idc.numel();
   TORCH_CHECK((size_t)dyc.numel() == tokens * (size_t)d);

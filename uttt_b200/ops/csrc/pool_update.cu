@@ -230,6 +230,8 @@ std::vector<at::Tensor> pool_step_fwd(at::Tensor m, at::Tensor d, double lr, int
   TORCH_CHECK(m.scalar_type() == at::kFloat && m.is_contiguous() && d.is_contiguous() && d.numel() == m.numel());
   const int D = m.size(-1);
   TORCH_CHECK(pool_step_supported(D));
+  m = dense16(m);
+  d = dense16(d);
   const long long rows = m.numel() / D;
   auto n = at::empty_like(m);
   auto w = at::empty(m.sizes(), m.options().dtype(at::kBFloat16));
@@ -259,16 +261,18 @@ std::vector<at::Tensor> pool_step_bwd(at::Tensor m, at::Tensor d, c10::optional<
   c10::cuda::CUDAGuard guard(m.device());
   const int D = m.size(-1);
   TORCH_CHECK(pool_step_supported(D) && m.is_contiguous() && d.is_contiguous());
+  m = dense16(m);
+  d = dense16(d);
   const long long rows = m.numel() / D;
   at::Tensor gnc, gwc;
   const float* gnp = nullptr;
   const __nv_bfloat16* gwp = nullptr;
   if (gn.has_value() && gn->defined()) {
-    gnc = gn->to(at::kFloat).contiguous();
+    gnc = dense16(gn->to(at::kFloat));
     gnp = gnc.data_ptr<float>();
   }
   if (gw.has_value() && gw->defined()) {
-    gwc = gw->to(at::kBFloat16).contiguous();
+    gwc = dense16(gw->to(at::kBFloat16));
     gwp = reinterpret_cast<const __nv_bfloat16*>(gwc.data_ptr());
   }
   auto gm = at::empty_like(m);
@@ -381,6 +385,7 @@ static dim3 frob_grid(long long per_matrix, int batch) {
 std::vector<at::Tensor> frob_normalize_fwd(at::Tensor g, double eps) {
   c10::cuda::CUDAGuard guard(g.device());
   TORCH_CHECK(g.dim() == 3 && g.is_contiguous() && (g.size(1) * g.size(2)) % 4 == 0);
+  g = dense16(g);
   const int batch = g.size(0);
   const long long per = (long long)g.size(1) * g.size(2);
   auto sumsq = at::zeros({batch}, g.options().dtype(at::kFloat));
@@ -405,7 +410,8 @@ std::vector<at::Tensor> frob_normalize_fwd(at::Tensor g, double eps) {
 at::Tensor frob_normalize_bwd(at::Tensor g, at::Tensor sumsq, at::Tensor dx, double eps) {
   c10::cuda::CUDAGuard guard(g.device());
   TORCH_CHECK(g.dim() == 3 && g.is_contiguous() && sumsq.scalar_type() == at::kFloat);
-  auto dxc = dx.to(at::kBFloat16).contiguous();
+  g = dense16(g);
+  auto dxc = dense16(dx.to(at::kBFloat16));
   const int batch = g.size(0);
   const long long per = (long long)g.size(1) * g.size(2);
   auto dot = at::zeros({batch}, sumsq.options());
