@@ -40,8 +40,9 @@ static inline int sm_count() { return at::cuda::getCurrentDeviceProperties()->mu
 // there are more), so that a warp works on 32 / G narrow rows at once: a head of 64 elements has 8 vectors, and one
 // such row per warp leaves three lanes of four idle and a quarter of the bytes in flight.  The row loops are
 // warp-uniform (a group past the end repeats the last row and stores nothing), so the shuffles see full warps.
-// 196,608 rows of 64: memory preprocessing 99 -> 16 us, its backward 248 -> 34, norm 32 -> 11, its backward 82 -> 22,
-// scatter 22 -> 8, gather 26 -> 10.  8192 rows of 192: preprocessing 7.2 -> 4.8 us, its backward 13.7 -> 9.3.
+// 196,608 rows of 64 (operands in L2, bf16): memory preprocessing 98 -> 16 us, its backward 250 -> 35, norm 31 -> 11, its
+// backward 91 -> 25, scatter 21 -> 8, gather 25 -> 9.  8192 rows of 192: preprocessing 7.0 -> 4.8 us, its backward
+// 15.6 -> 11.0.
 template <int G>
 __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
@@ -55,17 +56,20 @@ __device__ __forceinline__ float across_groups(float v) {
   for (int o = 16; o >= G; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+static inline int lanes_for(int vectors) { return vectors <= 4 ? 4 : vectors <= 8 ? 8 : vectors <= 16 ? 16 : 32; }
 template <typename F>
 static inline void with_lanes(int vectors, F&& f) {
-  if (vectors <= 4) f(std::integral_constant<int, 4>{});
-  else if (vectors <= 8) f(std::integral_constant<int, 8>{});
-  else if (vectors <= 16) f(std::integral_constant<int, 16>{});
-  else f(std::integral_constant<int, 32>{});
+  switch (lanes_for(vectors)) {
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    case 16: f(std::integral_constant<int, 16>{}); break;
+    default: f(std::integral_constant<int, 32>{});
+  }
 }
 
 // out[c] = sum over p of partial[p, c]: the per-block partial sums of a kernel.  32 columns per block, 32 row strands
-// each, so that a few hundred partial rows are a handful of loads in flight per thread: 4.2 us for 592 x 768, where the
-// general reduction took 15.7.
+// each, so that a few hundred partial rows are a handful of loads in flight per thread.  The norm's backward at
+// 8192 x 768, which sums 592 partial rows, went from 37.5 to 25.0 us with it in place of the general reduction.
 __global__ void __launch_bounds__(1024) col_sum_kernel(const float* __restrict__ partial, float* __restrict__ out, int rows,
                                                        long long cols) {
   __shared__ float part[32][33];
@@ -320,7 +324,7 @@ static std::vector<at::Tensor> rms_norm_bwd_impl(at::Tensor dy, at::Tensor x, c1
   auto dx = at::empty_like(x);
   at::Tensor wc, dw;
   const int nv = d / 8;
-  const int per_block = 4 * (nv <= 4 ? 8 : nv <= 8 ? 4 : nv <= 16 ? 2 : 1);      // 4 warps, 32 / G rows each
+  const int per_block = 4 * (32 / lanes_for(nv));
   int blocks = std::max(1, std::min((rows + per_block - 1) / per_block, sm_count() * 4));
   if (w.has_value() && w->defined()) {
     wc = dense16(w->to(x.scalar_type()));
@@ -593,9 +597,9 @@ __global__ void fw_qk_prep_bwd_kernel(const T* __restrict__ dy, const T* __restr
 }
 
 // Lane-group-per-(row, head) forms of the two kernels above, used when a head is at most 64 * MAXP 16-byte vectors wide
-// and half a rotary sub-head is a multiple of 8 elements.  G lanes hold a head (see "lane groups").  A lane owns pairs of vectors that are half a sub-head
-// apart, i.e. both members of eight rotary pairs: every access is a 16-byte vector, the head's values stay in
-// registers, the rotation needs no exchange, and the forward has no shared memory or block barrier.
+// and half a rotary sub-head is a multiple of 8 elements.  G lanes hold a head (see "lane groups").  A lane owns pairs of
+// vectors that are half a sub-head apart, i.e. both members of eight rotary pairs: every access is a 16-byte vector, the
+// head's values stay in registers, the rotation needs no exchange, and the forward has no shared memory or block barrier.
 struct QkPairMap {
   int nv, npairs, px, vps;
   __device__ __forceinline__ QkPairMap(int D, int rope_dim) {
@@ -1343,11 +1347,7 @@ static at::Tensor padded_buffer(int64_t rows_padded, int d, const at::TensorOpti
 }
 
 // rows of d elements that a block of 256 threads moves at a time
-static inline int copies_per_block(int d) {
-  int n = 0;
-  with_lanes(d / 8, [&](auto g) { n = 256 / decltype(g)::value; });
-  return n;
-}
+static inline int copies_per_block(int d) { return 256 / lanes_for(d / 8); }
 
 at::Tensor permute_rows(at::Tensor x, at::Tensor dest, int64_t rows_padded, c10::optional<at::Tensor> w,
                         c10::optional<at::Tensor> offsets, c10::optional<at::Tensor> sizes) {
@@ -1444,7 +1444,7 @@ __global__ void plan_count_kernel(const int* __restrict__ idx, int* __restrict__
 __global__ void plan_scan_kernel(int* __restrict__ blk_counts, int* __restrict__ sizes, int* __restrict__ offsets,
                                  int* __restrict__ tile_group, int B, int E, int nblk, int t_max) {
   // Latency-bound (one block, a few KB): the per-block counts of a group are fetched eight at a time, the group starts
-  // are a block-wide scan over 1024 groups at a time (256 groups: 16 -> 5 us).
+  // are a block-wide scan over 1024 groups at a time.  The plan of 4 x 49,152 rows over 64 experts: 22.3 -> 11.0 us.
   const int G = B * E;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ int warp_total[32];

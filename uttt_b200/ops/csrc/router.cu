@@ -10,9 +10,9 @@
 //   weight = alpha * probs[idx]   or   alpha * probs[idx] / sum_sel probs[idx]
 //   probs_sum[b, e] += probs[r, e]                            (load-balance statistics per sequence)
 //
-// Forward, bf16 rows: tensor cores (router_fwd_tc_kernel).  Other row types and shapes: a block stages 64 rows in shared memory, each warp multiplies 8 of them with lane = expert (two
-// experts per lane when E = 64) against the transposed router matrix in shared memory, then does the softmax
-// and the top-k with warp shuffles.
+// Forward, bf16 rows: tensor cores (router_fwd_tc_kernel).  Other row types and shapes: a block stages 64 rows in shared
+// memory, each warp multiplies 8 of them with lane = expert (two experts per lane when E = 64) against the transposed
+// router matrix in shared memory, then does the softmax and the top-k with warp shuffles.
 // Backward: one kernel turns (d weight, d probs_sum) into d logits and d rows (lane = slice of D), a second one
 // reduces d router = d logits^T . rows over row chunks with per-thread register tiles into per-block partials.
 // Reference behaviour: flame/custom_models/uttt_moe/moe_routing.py:7-75 (softmax router, selected_prob /
@@ -249,11 +249,11 @@ __global__ void __launch_bounds__(256) router_fwd_kernel(const T* __restrict__ r
 // accumulator of its own and the slabs are added in registers.  A thread owns a whole row of logits: softmax and top-k
 // need no shuffles.
 //   warp 8 / lane 0 : TMA producer, 64-column slabs of 128 rows -> ring
-//   warp 9 / lane 0 : MMA issuer, accumulators of two tiles in flight
+//   warp 9          : MMA issuer (an elected lane of the converged warp), accumulators of two tiles in flight
 //   warps 0-3, 4-7  : softmax, top-k and balance sums of every other tile, thread = row
 // One persistent block per SM; the three parts of the router stay in shared memory, swizzled as the B operand.  The
 // general kernel is bound by its fp32 multiply-adds and their shared-memory reads.
-// 196,608 rows of 64, 64 experts: 234 -> 28 us; 16,384 of 384, 32 experts: 45 -> 10.5 us; 4 of 192, 16 experts: 15 -> 6 us.
+// 196,608 rows of 64, 64 experts: 233 -> 28 us; 16,384 of 384, 32 experts: 45 -> 11 us; 4 of 192, 16 experts: 16 -> 7 us.
 // Relative error of the logits against 64 bits (general kernel): 0.8e-7 (1.4e-7), 0.9e-7 (3.5e-7), 1.0e-7 (2.7e-7); with
 // one accumulator for all slabs it was 1.1e-6 at 384 columns.
 constexpr int kRtStages = 4;

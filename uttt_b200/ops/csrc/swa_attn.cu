@@ -11,7 +11,8 @@
 //                     maximum that moves only when the running maximum exceeds it by 8 (log2 units); only then O is
 //                     rescaled in TMEM.
 //   warp 8 / lane 0 : TMA producer   K_j, V_j -> 128B-swizzled rings
-//   warp 9 / lane 0 : MMA issuer     per step and query tile: O += P_{j-1} V_{j-1}, then S_j = Q K_j^T
+//   warp 9          : MMA issuer     (an elected lane of the converged warp) per step and query tile:
+//                                    O += P_{j-1} V_{j-1}, then S_j = Q K_j^T
 // The two query tiles alternate: while the tensor core works for one, the other's softmax warps run, and each K/V tile
 // is fetched once for 256 queries.  Bound by the chain S -> softmax -> P -> MMA of a tile (tensor pipe a third busy,
 // exponential unit under half); a step of 128 keys pays its hand-overs once where a step of 64 paid them twice.

@@ -19,11 +19,13 @@
 //   swa_bwd_dq_out_kernel  fp32 dQ sums -> bf16, scaled
 // S, P and dS are formed once for all three gradients: five products and one exponential per element, where separate
 // dK/dV and dQ kernels needed seven and two.  The price is the addition of dQ in L2 (48 KB per tile at 96), in no fixed
-// order, to fp32 sums of b * h * ceil(lq, 128) * hd that are allocated and cleared on every call (50 MB at the size below).  Bound by the hand-overs between the products and the warps.  Measured with its preparation and
-// conversion: 785 -> 459 us at 4 x 16 heads x 96, 2048 queries on 4096 keys, window 2048.  With deterministic algorithms
-// asked for, the additions have an order: see launch_bwd.
+// order unless deterministic algorithms are asked for (see launch_bwd), to fp32 sums of b * h * ceil(lq, 128) * hd that
+// are allocated and cleared on every call: 50 MB at 4 x 16 heads x 96 with 2048 queries.
+// Bound by the hand-overs between the products and the warps.  Measured with its preparation and conversion:
+// 785 -> 459 us at that size on 4096 keys, window 2048.
 // Warps: 0-7 P and dS (two per TMEM lane quarter, each owning half of the 128 columns of a tile), 8-11 dQ,
-// 12 TMA producer lane, 13 MMA issuer lane.  Every wait is bounded (ptx::mbar_wait).
+// 12 TMA producer (one lane), 13 MMA issuer (an elected lane of the converged warp).
+// Every wait is bounded (ptx::mbar_wait).
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
